@@ -374,8 +374,10 @@ int ygx_traverse_finalize(int64_t total, int64_t num_internal, int64_t wf_capaci
  * split-list chunks; continuation queue.  needs_out (host, 14 uint64): what
  * each of them needed (re-run with at least these when
  * YGX_FLAG_LOG_OVERFLOW is set), then the most chunks one split list had,
- * the warp cycles spent on pieces and waiting, the pieces run, the 32-wide
- * steps run and the candidates those steps held.
+ * the warp cycles spent on pieces and waiting, the pieces run, the steps run
+ * and the candidates those steps held.  Unordered walks of at most 2^24
+ * nodes step over 64 candidates (the others over 32) and also queue
+ * num_internal + 1 whole targets.
  * flags_out also reports YGX_FLAG_TIMEOUT (a bounded wait gave up) and
  * YGX_FLAG_MALFORMED (a split list had more chunks than can be ordered);
  * with either flag the lists are not produced: use ygx_traverse_walk.

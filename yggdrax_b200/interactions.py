@@ -506,6 +506,14 @@ _TARGET_FALLBACK_WARNED: set = set()
 _LEARNED_TARGET_HINTS: dict = {}
 
 
+# Largest tree of the unordered walk over sibling pairs (24-bit slots).
+_PAIR_WALK_MAX_NODES = 1 << 24
+
+
+def _pair_walk(total: int, ordered: bool) -> bool:
+    return not ordered and total <= _PAIR_WALK_MAX_NODES
+
+
 def _target_caps(total: int, nl: int, hint) -> list:
     if hint is not None:
         return [max(1 << 16, int(1.15 * h * total) + 4096) for h in hint]
@@ -654,16 +662,26 @@ def _target_walk(topology, d, total, ni, nl, num_levels, center, radius, max_ext
                                overflow_entry_fraction=s["ovf_entries"] / entries)
     LAST_WALK_STATS.update(s, mode=mode_name, walk_runs=runs,
                            split_list_max_chunks=int(needs[8]),
-                           continuation_pieces=int(needs[7]), pieces_run=int(needs[11]),
+                           continuation_pieces=_continuation_pieces(needs, total, ni, ordered),
+                           pieces_run=int(needs[11]),
                            busy_fraction=int(needs[9]) / max(1, int(needs[9]) + int(needs[10])),
                            steps=int(needs[12]), far_records=int(needs[4]),
                            near_records=int(needs[5]),
-                           lane_fill=int(needs[13]) / max(1, 32 * int(needs[12])))
+                           lane_fill=int(needs[13]) / max(1, int(needs[12]) * (
+                               64 if _pair_walk(total, ordered) else 32)))
     if P == 0:
         node_offsets.zero_()
         level_offsets.zero_()
     return s, node_offsets, far_counts, level_offsets, sources, targets, target_levels, \
         near_offsets, near_counts, neighbors, nlp
+
+
+def _continuation_pieces(needs, total: int, ni: int, ordered: bool) -> int:
+    """Queue entries that are parts of a target: the unordered walk also
+    queues the root's children and one child of every other internal node."""
+    if not _pair_walk(total, ordered):
+        return int(needs[7])
+    return max(0, int(needs[7]) - (ni + 1))
 
 
 _DEVICE_BYTES: dict = {}
