@@ -76,12 +76,11 @@ def dual_tree_walk_mutual(left_child_full: torch.Tensor, right_child_full: torch
         L.ptr(near_a), L.ptr(near_b), counts.ctypes.data, flags.ctypes.data, gens.ctypes.data,
         L.ptr(ws), ws.numel(), L.stream_handle(dev)), "ygx_mutual_walk")
     f = int(flags[0])
-    b = lambda v: torch.tensor(bool(v), device=dev)  # noqa: E731
-    return MutualWalkResult(
-        far_a=far_a, far_b=far_b, far_count=torch.tensor(int(counts[0]), dtype=idt, device=dev),
-        near_a=near_a, near_b=near_b,
-        near_count=torch.tensor(int(counts[1]), dtype=idt, device=dev),
-        far_overflow=b(f & 1), near_overflow=b(f & 2), queue_overflow=b(f & 4))
+    n = torch.tensor([int(counts[0]), int(counts[1])], dtype=idt).to(dev)
+    over = torch.tensor([bool(f & 1), bool(f & 2), bool(f & 4)]).to(dev)
+    return MutualWalkResult(far_a=far_a, far_b=far_b, far_count=n[0], near_a=near_a,
+                            near_b=near_b, near_count=n[1], far_overflow=over[0],
+                            near_overflow=over[1], queue_overflow=over[2])
 
 
 __all__ = ["MutualWalkResult", "dual_tree_walk_mutual"]
