@@ -206,10 +206,12 @@ def require_cuda(t: torch.Tensor, what: str = "input") -> torch.device:
     return t.device
 
 
-def workspace(nbytes: int, device: torch.device) -> torch.Tensor:
-    """Device workspace with a zeroed status header."""
+def workspace(nbytes: int, device: torch.device, zero: bool = True) -> torch.Tensor:
+    """Device workspace with a zeroed status header (zero=False: for entry
+    points that clear their own, or have none)."""
     ws = torch.empty(max(int(nbytes), 512), dtype=torch.uint8, device=device)
-    ws[:512].zero_()
+    if zero:
+        ws[:512].zero_()
     return ws
 
 

@@ -324,7 +324,6 @@ __global__ void __launch_bounds__(kMomThreads)
   __shared__ Tables tb;
   __shared__ float raw[kMomNodes][kMomPad], pk[kMomNodes][kMomPad];
   __shared__ float pw[kMomNodes][3][kMaxOrder + 1];
-  __shared__ float com[kMomNodes][3], ctr[kMomNodes][3];
   __shared__ float trace[kMomNodes], r2rk[kMomNodes][3], r2[kMomNodes][9], r4[kMomNodes];
   __shared__ int odd[kMomNodes];   // a sum is infinite or NaN
   __shared__ int64_t rng[kMomNodes][2];
@@ -358,12 +357,10 @@ __global__ void __launch_bounds__(kMomThreads)
       const float m = raw[v][0];
       const float cm =
           (Ccols < 4 || m == 0.0f) ? 0.0f : __fdiv_rn(raw[v][3 - ax], m == 0.0f ? 1.0f : m);
-      com[v][ax] = cm;
       if (o_com) o_com[3 * q0 + x] = cm;
       if (ax == 0) o_mass[q0 + v] = m;
       if (o_packed) {
         const float ct = centers ? centers[3 * q0 + x] : cm;
-        ctr[v][ax] = ct;
         o_center[3 * q0 + x] = ct;
         powers(-ct, pw[v][ax]);
       }

@@ -161,6 +161,8 @@ __global__ void k_pw_slots(const float* __restrict__ center, const float* __rest
                            const int32_t* __restrict__ near_rcap,
                            const int64_t* __restrict__ pad_far,
                            const int64_t* __restrict__ pad_near, PwRow* __restrict__ rows,
+                           unsigned* __restrict__ first_ovf_far,
+                           unsigned* __restrict__ first_ovf_near,
                            uint32_t* __restrict__ status) {
   for (int32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < total;
        s += gridDim.x * blockDim.x) {
@@ -168,6 +170,7 @@ __global__ void k_pw_slots(const float* __restrict__ center, const float* __rest
     if (far_rcap) {
       f.pad = pad_far[s];
       f.rcap = far_rcap[s];
+      first_ovf_far[s] = 0xffffffffu;
     }
     rows[s] = f;
     if (s >= ni) {
@@ -176,6 +179,7 @@ __global__ void k_pw_slots(const float* __restrict__ center, const float* __rest
       if (far_rcap) {
         q.pad = pad_near[lp];
         q.rcap = near_rcap[lp];
+        first_ovf_near[lp] = 0xffffffffu;
       }
       rows[total + s - ni] = q;
     }

@@ -41,8 +41,10 @@
 // then targets in level order, and wait (bounded) only on a parent that is
 // still in progress.  (Unordered walks of trees up to 2^24 nodes run
 // pair_walk.cuh instead: the same pairs in cheaper steps.)
+#include <string.h>
+
 #include "rows.cuh"
-#include "scan.cuh"
+#include "scan_seg.cuh"
 #include "sort.cuh"
 
 namespace ygx {
@@ -1017,34 +1019,52 @@ __global__ void __launch_bounds__(kTwThreads, kTwBlocksPerSM) k_tw_walk(TwArgs a
 // ---------------------------------------------------------------------------
 // statistics and assembly
 
-// Row totals and maxima (far per node, near per leaf position).
+// Row totals and maxima (far per node, near per leaf position); with predicted
+// rows also the rows that outgrew their capacity, the entries past the
+// capacities and the entries those rows hold (their extension).  out: far
+// total, near total, far max, near max, ovf rows, ovf entries, far extension,
+// near extension.  The tree's level offsets go along, so that the host reads
+// one block.
 __global__ void k_tw_row_stats(const int32_t* __restrict__ far_cnt, int32_t total,
                                const int32_t* __restrict__ near_cnt, int32_t L,
+                               const int32_t* __restrict__ far_rcap,
+                               const int32_t* __restrict__ near_rcap, const void* level_offsets,
+                               int index_bits, int num_levels, int64_t* __restrict__ levels_out,
                                unsigned long long* __restrict__ out) {
-  unsigned long long fs = 0, ns = 0, fm = 0, nm = 0;
+  if (blockIdx.x == 0 && (int)threadIdx.x <= num_levels)
+    levels_out[threadIdx.x] = load_idx(level_offsets, index_bits, threadIdx.x);
+  unsigned long long v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   for (int32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < total; k += gridDim.x * blockDim.x) {
-    const unsigned long long v = (unsigned long long)far_cnt[k];
-    fs += v;
-    fm = v > fm ? v : fm;
+    const unsigned long long c = (unsigned long long)far_cnt[k];
+    v[0] += c;
+    v[2] = c > v[2] ? c : v[2];
+    if (far_rcap && (long long)c > far_rcap[k]) {
+      v[4] += 1;
+      v[5] += c - (unsigned long long)far_rcap[k];
+      v[6] += c;
+    }
     if (k < L) {
       const unsigned long long w = (unsigned long long)near_cnt[k];
-      ns += w;
-      nm = w > nm ? w : nm;
+      v[1] += w;
+      v[3] = w > v[3] ? w : v[3];
+      if (far_rcap && (long long)w > near_rcap[k]) {
+        v[4] += 1;
+        v[5] += w - (unsigned long long)near_rcap[k];
+        v[7] += w;
+      }
     }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    fs += __shfl_xor_sync(0xffffffffu, fs, o);
-    ns += __shfl_xor_sync(0xffffffffu, ns, o);
-    const unsigned long long x = __shfl_xor_sync(0xffffffffu, fm, o);
-    const unsigned long long y = __shfl_xor_sync(0xffffffffu, nm, o);
-    fm = x > fm ? x : fm;
-    nm = y > nm ? y : nm;
-  }
-  if ((threadIdx.x & 31) == 0) {
-    if (fs) atomicAdd(&out[0], fs);
-    if (ns) atomicAdd(&out[1], ns);
-    atomicMax(&out[2], fm);
-    atomicMax(&out[3], nm);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long x = __shfl_xor_sync(0xffffffffu, v[q], o);
+      if (q == 2 || q == 3) v[q] = x > v[q] ? x : v[q];
+      else v[q] += x;
+    }
+    if ((threadIdx.x & 31) == 0 && v[q]) {
+      if (q == 2 || q == 3) atomicMax(&out[q], v[q]);
+      else atomicAdd(&out[q], v[q]);
+    }
   }
 }
 
@@ -1084,11 +1104,26 @@ __global__ void __launch_bounds__(256)
 // entries to the row's raw area at base[row] + the chunk's offset within
 // the row (record key: row << 32 | offset); the rows are sorted afterwards.
 // A record that does not fit its row or its pool is reported, not copied.
+struct TwCopy {
+  const unsigned long long* keys;
+  const TwChunk* recs;
+  int64_t m;
+  const int64_t* base;
+  int64_t rows;
+  const int32_t* pool;
+  int64_t pool_cap;
+  int32_t* raw;
+  int64_t raw_cap;
+};
 __global__ void __launch_bounds__(256)
-    k_tw_copy_raw(const unsigned long long* __restrict__ keys, const TwChunk* __restrict__ recs,
-                  int64_t m, const int64_t* __restrict__ base, int64_t rows,
-                  const int32_t* __restrict__ pool, int64_t pool_cap, int32_t* __restrict__ raw,
-                  int64_t raw_cap, uint32_t* __restrict__ status) {
+    k_tw_copy_raw(const TwCopy far, const TwCopy near_, uint32_t* __restrict__ status) {
+  const TwCopy& q = blockIdx.y == 0 ? far : near_;
+  const unsigned long long* __restrict__ keys = q.keys;
+  const TwChunk* __restrict__ recs = q.recs;
+  const int64_t* __restrict__ base = q.base;
+  const int32_t* __restrict__ pool = q.pool;
+  int32_t* __restrict__ raw = q.raw;
+  const int64_t m = q.m, rows = q.rows, pool_cap = q.pool_cap, raw_cap = q.raw_cap;
   const int lane = threadIdx.x & 31;
   const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -1109,62 +1144,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Predicted rows: per list, the rows that outgrew their capacity, the
-// entries past the capacities and the entries those rows hold (their
-// extension).  out: ovf rows, ovf entries, far extension, near extension.
-__global__ void k_tw_ext_stats(const int32_t* __restrict__ far_cnt,
-                               const int32_t* __restrict__ far_rcap, int32_t total,
-                               const int32_t* __restrict__ near_cnt,
-                               const int32_t* __restrict__ near_rcap, int32_t L,
-                               unsigned long long* __restrict__ out) {
-  unsigned long long rows = 0, past = 0, ef = 0, en = 0;
-  for (int32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < total; k += gridDim.x * blockDim.x) {
-    const int32_t c = far_cnt[k], r = far_rcap[k];
-    if (c > r) {
-      ++rows;
-      past += (unsigned long long)(c - r);
-      ef += (unsigned long long)c;
-    }
-    if (k < L) {
-      const int32_t cn = near_cnt[k], rn = near_rcap[k];
-      if (cn > rn) {
-        ++rows;
-        past += (unsigned long long)(cn - rn);
-        en += (unsigned long long)cn;
-      }
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    rows += __shfl_xor_sync(0xffffffffu, rows, o);
-    past += __shfl_xor_sync(0xffffffffu, past, o);
-    ef += __shfl_xor_sync(0xffffffffu, ef, o);
-    en += __shfl_xor_sync(0xffffffffu, en, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    if (rows) atomicAdd(&out[0], rows);
-    if (past) atomicAdd(&out[1], past);
-    if (ef) atomicAdd(&out[2], ef);
-    if (en) atomicAdd(&out[3], en);
-  }
-}
-
-// Extension length of every row: its count if it outgrew the capacity.
-__global__ void k_tw_ext_len(const int32_t* __restrict__ cnt, const int32_t* __restrict__ rcap,
-                             int32_t rows, int32_t* __restrict__ ext_len) {
-  for (int32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < rows; k += gridDim.x * blockDim.x)
-    ext_len[k] = cnt[k] > rcap[k] ? cnt[k] : 0;
-}
-
-// Where every row's raw entries sit: its padded slot, or for a row that
-// outgrew it, its extension behind all padded slots.
-__global__ void k_tw_roff(const int32_t* __restrict__ cnt, const int32_t* __restrict__ rcap,
-                          const int64_t* __restrict__ pad, const int64_t* __restrict__ ext_off,
-                          int32_t rows, int64_t* __restrict__ roff) {
-  const int64_t pad_total = pad[rows];
-  for (int32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < rows; k += gridDim.x * blockDim.x)
-    roff[k] = cnt[k] > rcap[k] ? pad_total + ext_off[k] : pad[k];
-}
-
 // A row that outgrew its slot: the entries written in place (offsets below
 // the first one that went to the pool) move to the front of its extension.
 // The extensions lie back to back behind all slots (ext_off: exclusive sums
@@ -1183,11 +1162,25 @@ __device__ __forceinline__ int32_t tw_row_of(const int64_t* __restrict__ ext_off
   }
   return lo;
 }
-__global__ void k_tw_prefix_copy(const int32_t* __restrict__ cnt, const int64_t* __restrict__ pad,
-                                 const unsigned* __restrict__ first_ovf,
-                                 const int64_t* __restrict__ ext_off, int32_t rows,
-                                 int32_t* __restrict__ raw, int64_t raw_cap,
+struct TwPrefix {
+  const int32_t* cnt;
+  const int64_t* pad;
+  const unsigned* first_ovf;
+  const int64_t* ext_off;
+  int32_t rows;
+  int32_t* raw;
+  int64_t raw_cap;
+};
+__global__ void k_tw_prefix_copy(const TwPrefix far, const TwPrefix near_,
                                  uint32_t* __restrict__ status) {
+  const TwPrefix& q = blockIdx.y == 0 ? far : near_;
+  const int32_t* __restrict__ cnt = q.cnt;
+  const int64_t* __restrict__ pad = q.pad;
+  const unsigned* __restrict__ first_ovf = q.first_ovf;
+  const int64_t* __restrict__ ext_off = q.ext_off;
+  int32_t* __restrict__ raw = q.raw;
+  const int32_t rows = q.rows;
+  const int64_t raw_cap = q.raw_cap;
   const int lane = threadIdx.x & 31;
   const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -1215,54 +1208,103 @@ __global__ void k_tw_prefix_copy(const int32_t* __restrict__ cnt, const int64_t*
   }
 }
 
-// counts in nodes_by_level order; far offsets; index-dtype tables
-__global__ void k_tw_gather(const int32_t* __restrict__ cnt, const int32_t* __restrict__ nbl,
-                            int32_t m, int32_t* __restrict__ out) {
-  for (int32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < m; r += gridDim.x * blockDim.x)
-    out[r] = cnt[nbl[r]];
-}
-__global__ void k_tw_far_tables(const int64_t* __restrict__ obl, const int32_t* __restrict__ nbl,
-                                const int32_t* __restrict__ cnt, int32_t total, int index_bits,
-                                void* node_offsets, void* counts_out, const void* tree_level_offsets,
-                                int num_levels, void* level_offsets_out,
-                                int64_t* __restrict__ off_node) {
-  for (int32_t r = blockIdx.x * blockDim.x + threadIdx.x; r <= total; r += gridDim.x * blockDim.x) {
-    if (r == total) {
-      store_idx(node_offsets, index_bits, total, obl[total]);
-      if (off_node) off_node[total] = obl[total];
+// The lists' plan (scan_seg.cuh): far rows in level order, near rows, and with
+// predicted rows the extensions of the rows that outgrew their slots -- offset
+// and count tables in the index dtype, and where every raw row sits: its
+// slot, or its extension behind all slots.
+struct TwPlan {
+  const int32_t *far_cnt, *near_cnt, *far_rcap, *near_rcap, *nbl;
+  const int64_t *pad_far, *pad_near;
+  int64_t total, L;
+  const void* tree_level_offsets;
+  int num_levels, index_bits;
+  void *node_offsets, *far_counts, *level_offsets, *near_offsets, *near_counts;
+  int64_t *off_node, *near_off, *ext_far, *ext_near, *roff_far, *roff_near;
+
+  __device__ int64_t n(int s) const { return s == 0 || s == 2 ? total : L; }
+  __device__ int64_t get(int s, int64_t i) const {
+    if (s == 0) return far_cnt[nbl[i]];
+    if (s == 1) return near_cnt[i];
+    const int32_t c = s == 2 ? far_cnt[i] : near_cnt[i];
+    return c > (s == 2 ? far_rcap[i] : near_rcap[i]) ? c : 0;
+  }
+  // level l starts at rank tree_level_offsets[l] (non-decreasing)
+  __device__ void levels(int64_t rank, int64_t p) const {
+    int lo = 0, hi = num_levels + 1;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (load_idx(tree_level_offsets, index_bits, mid) < rank) lo = mid + 1;
+      else hi = mid;
+    }
+    for (; lo <= num_levels && load_idx(tree_level_offsets, index_bits, lo) == rank; ++lo)
+      store_idx(level_offsets, index_bits, lo, p);
+  }
+  __device__ void put(int s, int64_t i, int64_t p, int64_t v) const {
+    if (s == 0) {
+      const int32_t node = nbl[i];
+      store_idx(node_offsets, index_bits, node, p);
+      store_idx(far_counts, index_bits, node, v);
+      if (off_node) off_node[node] = p;
+      levels(i, p);
+    } else if (s == 1) {
+      near_off[i] = p;
+      store_idx(near_offsets, index_bits, i, p);
+      store_idx(near_counts, index_bits, i, v);
+    } else if (s == 2) {
+      ext_far[i] = p;
+      roff_far[i] = v > 0 ? pad_far[total] + p : pad_far[i];
     } else {
-      const int32_t v = nbl[r];
-      store_idx(node_offsets, index_bits, v, obl[r]);
-      if (off_node) off_node[v] = obl[r];
-      store_idx(counts_out, index_bits, v, cnt[v]);
-    }
-    if (r <= num_levels) {
-      const int64_t li = load_idx(tree_level_offsets, index_bits, r);
-      store_idx(level_offsets_out, index_bits, r, obl[li]);
+      ext_near[i] = p;
+      roff_near[i] = v > 0 ? pad_near[L] + p : pad_near[i];
     }
   }
-}
-__global__ void k_tw_near_tables(const int64_t* __restrict__ off, const int32_t* __restrict__ cnt,
-                                 int32_t L, int index_bits, void* offsets_out, void* counts_out) {
-  for (int32_t j = blockIdx.x * blockDim.x + threadIdx.x; j <= L; j += gridDim.x * blockDim.x) {
-    store_idx(offsets_out, index_bits, j, off[j]);
-    if (j < L) store_idx(counts_out, index_bits, j, cnt[j]);
+  __device__ void end(int s, int64_t t) const {
+    if (s == 0) {
+      store_idx(node_offsets, index_bits, total, t);
+      if (off_node) off_node[total] = t;
+      levels(total, t);
+    } else if (s == 1) {
+      near_off[L] = t;
+      store_idx(near_offsets, index_bits, L, t);
+    } else if (s == 2) {
+      ext_far[total] = t;
+    } else {
+      ext_near[L] = t;
+    }
   }
-}
+};
+
+// Predicted rows' slots: exclusive sums of the capacities, and their totals.
+struct TwPad {
+  const int32_t *far_rcap, *near_rcap;
+  int64_t total, L;
+  int64_t *pad_far, *pad_near, *sums;
+  __device__ int64_t n(int s) const { return s == 0 ? total : L; }
+  __device__ int64_t get(int s, int64_t i) const { return s == 0 ? far_rcap[i] : near_rcap[i]; }
+  __device__ void put(int s, int64_t i, int64_t p, int64_t) const {
+    (s == 0 ? pad_far : pad_near)[i] = p;
+  }
+  __device__ void end(int s, int64_t t) const {
+    (s == 0 ? pad_far : pad_near)[s == 0 ? total : L] = t;
+    sums[s] = t;
+  }
+};
 
 // Dense neighbour leaf positions (L x max_nbr, -1 padded) of
 // _result_to_neighbors (:3658-3688).
+// One warp per row: no division, whole sectors written.  263,480 rows of 98
+// (the 4,194,304-particle fixed-depth octree): 130 -> 94 us.
 __global__ void k_tw_nbr_leaf_pos(const int64_t* __restrict__ near_off,
                                   const int32_t* __restrict__ near_cnt, int64_t L,
                                   const void* neighbors, int index_bits,
                                   const int32_t* __restrict__ leafpos, int64_t max_nbr, void* out) {
-  const int64_t n = L * max_nbr;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t j = e / max_nbr, k = e - j * max_nbr;
-    int64_t v = -1;
-    if (k < near_cnt[j]) v = leafpos[load_idx(neighbors, index_bits, near_off[j] + k)];
-    store_idx(out, index_bits, e, v);
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < L; j += nw) {
+    const int64_t off = near_off[j], cnt = near_cnt[j], o = j * max_nbr;
+    for (int64_t k = lane; k < max_nbr; k += 32)
+      store_idx(out, index_bits, o + k,
+                k < cnt ? leafpos[load_idx(neighbors, index_bits, off + k)] : -1);
   }
 }
 
@@ -1279,7 +1321,8 @@ struct TwScratch {
   uint32_t* status;
   TwCtl* ctl;
   unsigned int* gen_hist;
-  unsigned long long* rowstat;  // 4 words
+  unsigned long long* rowstat;  // 8 words
+  int64_t* levels;              // the tree's level offsets, for the host
   TwRec* recs;
   int32_t* first;
   int32_t* rank;
@@ -1315,8 +1358,6 @@ struct TwScratch {
   int32_t* sorted_cnt;
   int64_t* dest;
   int64_t* scan_tmp;
-  int32_t* cnt_by_level;
-  int64_t* obl;
   int64_t* near_off;
   void* sort_ws;
   size_t sort_ws_bytes;
@@ -1324,8 +1365,8 @@ struct TwScratch {
   int64_t* far_off_node;
   unsigned* first_ovf_far;  // predicted rows
   unsigned* first_ovf_near;
-  int32_t* ext_len;
-  int64_t* ext_off;
+  int64_t* ext_far;
+  int64_t* ext_near;
   int64_t* roff_far;
   int64_t* roff_near;
   RowSortScratch rs;
@@ -1344,6 +1385,7 @@ static TwScratch carve_tw(Arena& a, int64_t total, int64_t L, const TwCaps& c, b
   s.ctl = a.take<TwCtl>(1);
   s.gen_hist = a.take<unsigned int>(kTwHist);
   s.rowstat = a.take<unsigned long long>(8);
+  s.levels = a.take<int64_t>(kTwHist / 2 + 1);
   // per node, zeroed: split counts, insertion points, chunk counts, pieces
   s.s_cnt = a.take<int32_t>(total);
   s.s_ins = a.take<int32_t>(total);
@@ -1351,6 +1393,7 @@ static TwScratch carve_tw(Arena& a, int64_t total, int64_t L, const TwCaps& c, b
   s.pieces_left = a.take<int32_t>(total);
   s.far_cnt = a.take<int32_t>(total);
   s.near_cnt = a.take<int32_t>(L > 0 ? L : 1);
+  s.q_ready = a.take<unsigned int>(c.queue);
   // per node, written before use
   s.s_head = a.take<int32_t>(total);
   if (pairs) {
@@ -1370,7 +1413,6 @@ static TwScratch carve_tw(Arena& a, int64_t total, int64_t L, const TwCaps& c, b
     s.spill = a.take<unsigned long long>(c.spill);
     s.queue = a.take<TwPiece>(c.queue);
   }
-  s.q_ready = a.take<unsigned int>(c.queue);
   s.far_pool = a.take<int32_t>(c.far);
   s.near_pool = a.take<int32_t>(c.near_);
   s.far_keys = a.take<unsigned long long>(c.far_rec);
@@ -1383,25 +1425,22 @@ static TwScratch carve_tw(Arena& a, int64_t total, int64_t L, const TwCaps& c, b
   s.keys_sorted = a.take<unsigned long long>(mrec);
   s.sorted_cnt = a.take<int32_t>(mrec);
   s.dest = a.take<int64_t>(mrec + 1);
-  const int64_t scan_n = mrec > total ? mrec : total;
-  s.scan_tmp = a.take<int64_t>(scan_scratch_elems(scan_n));
-  s.cnt_by_level = a.take<int32_t>(total);
-  s.obl = a.take<int64_t>(total + 1);
+  const size_t plan = seg_scan_elems(total, 4);
+  const size_t chunks = scan_scratch_elems(mrec);
+  s.scan_tmp = a.take<int64_t>(plan > chunks ? plan : chunks);
   s.near_off = a.take<int64_t>((L > 0 ? L : 1) + 1);
   s.sort_ws_bytes = onesweep_scratch_bytes(mrec) + 256;
   s.sort_ws = a.take<unsigned char>(s.sort_ws_bytes);
   s.far_off_node = nullptr;
   s.first_ovf_far = s.first_ovf_near = nullptr;
-  s.ext_len = nullptr;
-  s.ext_off = s.roff_far = s.roff_near = nullptr;
+  s.ext_far = s.ext_near = s.roff_far = s.roff_near = nullptr;
   s.rs = RowSortScratch{nullptr, nullptr, nullptr, nullptr, 0};
   if (!ordered) {
-    const int64_t mx = (total > L ? total : L) + 1;
     s.far_off_node = a.take<int64_t>(total + 1);
     s.first_ovf_far = a.take<unsigned>(total);
     s.first_ovf_near = a.take<unsigned>(L > 0 ? L : 1);
-    s.ext_len = a.take<int32_t>(mx);
-    s.ext_off = a.take<int64_t>(mx);
+    s.ext_far = a.take<int64_t>(total + 1);
+    s.ext_near = a.take<int64_t>((L > 0 ? L : 1) + 1);
     s.roff_far = a.take<int64_t>(total);
     s.roff_near = a.take<int64_t>(L > 0 ? L : 1);
     s.rs = carve_row_sort(a, total, L);
@@ -1459,11 +1498,10 @@ int ygx_target_walk(const float* center, const float* radius, const float* max_e
   const int64_t L = total - num_internal;
   Arena ar{(char*)ws, 0, ws_bytes};
   TwScratch s = carve_tw(ar, total, L, c, ordered != 0);
-  const size_t zero_bytes = (size_t)((char*)(s.near_cnt + (L > 0 ? L : 1)) - (char*)s.status);
-  if (cudaMemsetAsync(s.status, 0, zero_bytes, stream) != cudaSuccess ||
-      cudaMemsetAsync(s.q_ready, 0, sizeof(unsigned int) * c.queue, stream) != cudaSuccess)
-    return YGX_ERR_CUDA;
-  if (pred && (cudaMemsetAsync(s.first_ovf_far, 0xff, sizeof(unsigned) * total, stream) !=
+  const bool pairs = use_pairs(total, ordered != 0);
+  const size_t zero_bytes = (size_t)((char*)(s.q_ready + c.queue) - (char*)s.status);
+  if (cudaMemsetAsync(s.status, 0, zero_bytes, stream) != cudaSuccess) return YGX_ERR_CUDA;
+  if (pred && !pairs && (cudaMemsetAsync(s.first_ovf_far, 0xff, sizeof(unsigned) * total, stream) !=
                    cudaSuccess ||
                cudaMemsetAsync(s.first_ovf_near, 0xff, sizeof(unsigned) * (L > 0 ? L : 1),
                                stream) != cudaSuccess))
@@ -1486,11 +1524,11 @@ int ygx_target_walk(const float* center, const float* radius, const float* max_e
     blk_records = (unsigned)(br < 4 ? 4 : (br > 64 ? 64 : br));
   }
   cudaError_t e = cudaSuccess;
-  if (use_pairs(total, ordered != 0)) {
+  if (pairs) {
     k_pw_slots<<<grid_for(total, 256), 256, 0, stream>>>(
         center, radius, max_extent, left32, right32, NI, T, root, mac, dehnen_radius_scale, s.sc,
         s.sid, s.queue32, s.q_ready, s.ctl, leafpos32, far_rcap32, near_rcap32, pad_far, pad_near,
-        s.pw_rows, s.status);
+        s.pw_rows, s.first_ovf_far, s.first_ovf_near, s.status);
     YGX_CHECK_LAUNCH();
     PwArgs a;
     a.sc = s.sc;
@@ -1639,37 +1677,34 @@ int ygx_target_walk(const float* center, const float* radius, const float* max_e
   }
   if (e != cudaSuccess) return YGX_ERR_CUDA;
   YGX_CHECK_LAUNCH();
-  k_tw_row_stats<<<grid_for(total, 256, kNumSMs * 4), 256, 0, stream>>>(s.far_cnt, T, s.near_cnt,
-                                                                       (int32_t)L, s.rowstat);
+  k_tw_row_stats<<<grid_for(total, 256, kNumSMs * 4), 256, 0, stream>>>(
+      s.far_cnt, T, s.near_cnt, (int32_t)L, pred ? far_rcap32 : nullptr,
+      pred ? near_rcap32 : nullptr, tree_level_offsets, index_bits, num_levels, s.levels,
+      s.rowstat);
   YGX_CHECK_LAUNCH();
-  if (pred) {
-    k_tw_ext_stats<<<grid_for(total, 256, kNumSMs * 4), 256, 0, stream>>>(
-        s.far_cnt, far_rcap32, T, s.near_cnt, near_rcap32, (int32_t)L, s.rowstat + 4);
-    YGX_CHECK_LAUNCH();
-  }
+  // status word, control block, histogram, row statistics and levels lie one
+  // behind the other: one read
+  alignas(16) char block[8192];
+  const char* first = (const char*)s.status;
+  const size_t bytes = (const char*)(s.levels + kTwHist / 2 + 1) - first;
+  if (bytes > sizeof(block)) return YGX_ERR_ARG;
+  if (cudaMemcpyAsync(block, first, bytes, cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+      cudaStreamSynchronize(stream) != cudaSuccess)
+    return YGX_ERR_CUDA;
+  auto at = [&](const void* p) { return block + ((const char*)p - first); };
   TwCtl ctl;
   unsigned int hist[kTwHist];
   unsigned long long rs[8];
   int64_t lvl_off[kTwHist / 2 + 1];
-  int32_t lvl_off32[kTwHist / 2 + 1];
-  const bool i64 = index_bits == 64;
-  if (cudaMemcpyAsync(i64 ? (void*)lvl_off : (void*)lvl_off32, tree_level_offsets,
-                      (size_t)(num_levels + 1) * (i64 ? 8 : 4), cudaMemcpyDeviceToHost,
-                      stream) != cudaSuccess ||
-      cudaMemcpyAsync(&ctl, s.ctl, sizeof(TwCtl), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
-      cudaMemcpyAsync(hist, s.gen_hist, sizeof(hist), cudaMemcpyDeviceToHost, stream) !=
-          cudaSuccess ||
-      cudaMemcpyAsync(rs, s.rowstat, sizeof(rs), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
-      cudaMemcpyAsync(flags_out, s.status, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream) !=
-          cudaSuccess ||
-      cudaStreamSynchronize(stream) != cudaSuccess)
-    return YGX_ERR_CUDA;
+  memcpy(flags_out, at(s.status), sizeof(uint32_t));
+  memcpy(&ctl, at(s.ctl), sizeof(ctl));
+  memcpy(hist, at(s.gen_hist), sizeof(hist));
+  memcpy(rs, at(s.rowstat), sizeof(rs));
+  memcpy(lvl_off, at(s.levels), sizeof(int64_t) * (num_levels + 1));
   // generations: every node's self pair {v, v} sits at generation depth(v);
   // every other pair was evaluated once from each side
   unsigned long long wf2[kTwHist];
   for (int g = 0; g < kTwHist; ++g) wf2[g] = hist[g];
-  if (!i64)
-    for (int l = 0; l <= num_levels; ++l) lvl_off[l] = lvl_off32[l];
   for (int l = 0; l < num_levels && l < kTwHist; ++l)
     wf2[l] += 2ull * (unsigned long long)(lvl_off[l + 1] - lvl_off[l]);
   unsigned long long mw = 1, gens = 0;
@@ -1746,20 +1781,14 @@ int ygx_target_walk_lists(int64_t total, int64_t num_internal, const int64_t* ca
   Arena ar{(char*)ws, 0, ws_bytes};
   TwScratch s = carve_tw(ar, total, L, c, ordered != 0);
   const int32_t T = (int32_t)total;
-  // offset / count tables
-  k_tw_gather<<<grid_for(total, 256), 256, 0, stream>>>(s.far_cnt, nbl32, T, s.cnt_by_level);
-  YGX_CHECK_LAUNCH();
-  int rc = exclusive_scan<int32_t>(s.cnt_by_level, total, s.obl, s.scan_tmp, stream);
+  // offset / count tables and where the raw rows sit
+  const TwPlan plan{s.far_cnt,  s.near_cnt,   far_rcap32,   near_rcap32,  nbl32,
+                    pad_far,    pad_near,     total,        L,            tree_level_offsets,
+                    num_levels, index_bits,   node_offsets, far_counts,   level_offsets,
+                    near_offsets, near_counts, s.far_off_node, s.near_off, s.ext_far,
+                    s.ext_near, s.roff_far,   s.roff_near};
+  int rc = seg_scan(plan, total, pred ? 4 : 2, s.scan_tmp, stream);
   if (rc) return rc;
-  k_tw_far_tables<<<grid_for(total + 1, 256), 256, 0, stream>>>(
-      s.obl, nbl32, s.far_cnt, T, index_bits, node_offsets, far_counts, tree_level_offsets,
-      num_levels, level_offsets, s.far_off_node);
-  YGX_CHECK_LAUNCH();
-  rc = exclusive_scan<int32_t>(s.near_cnt, L, s.near_off, s.scan_tmp, stream);
-  if (rc) return rc;
-  k_tw_near_tables<<<grid_for(L + 1, 256), 256, 0, stream>>>(s.near_off, s.near_cnt, (int32_t)L,
-                                                            index_bits, near_offsets, near_counts);
-  YGX_CHECK_LAUNCH();
   if (!ordered) {
     // chunks straight to their rows (offsets taken by the walk), then every
     // row sorted.  Rows sit at their output offsets, or with predicted
@@ -1769,38 +1798,24 @@ int ygx_target_walk_lists(int64_t total, int64_t num_internal, const int64_t* ca
     const int64_t* far_base = s.far_off_node;
     const int64_t* near_base = s.near_off;
     if (pred) {
-      for (int pass = 0; pass < 2; ++pass) {
-        const bool far = pass == 0;
-        const int32_t rows = far ? T : LL;
-        const int32_t* cnt = far ? s.far_cnt : s.near_cnt;
-        const int32_t* rcap = far ? far_rcap32 : near_rcap32;
-        const int64_t* pad = far ? pad_far : pad_near;
-        int64_t* roff = far ? s.roff_far : s.roff_near;
-        if (rows == 0) continue;
-        k_tw_ext_len<<<grid_for(rows, 256), 256, 0, stream>>>(cnt, rcap, rows, s.ext_len);
-        YGX_CHECK_LAUNCH();
-        rc = exclusive_scan<int32_t>(s.ext_len, rows, s.ext_off, s.scan_tmp, stream);
-        if (rc) return rc;
-        k_tw_roff<<<grid_for(rows, 256), 256, 0, stream>>>(cnt, rcap, pad, s.ext_off, rows, roff);
-        YGX_CHECK_LAUNCH();
-        k_tw_prefix_copy<<<kNumSMs * 8, 256, 0, stream>>>(
-            cnt, pad, far ? s.first_ovf_far : s.first_ovf_near, s.ext_off, rows,
-            far ? far_raw : near_raw, far ? far_raw_cap : near_raw_cap, s.status);
-        YGX_CHECK_LAUNCH();
-      }
+      k_tw_prefix_copy<<<dim3(kNumSMs * 8, 2), 256, 0, stream>>>(
+          TwPrefix{s.far_cnt, pad_far, s.first_ovf_far, s.ext_far, T, far_raw, far_raw_cap},
+          TwPrefix{s.near_cnt, pad_near, s.first_ovf_near, s.ext_near, LL, near_raw,
+                   near_raw_cap},
+          s.status);
+      YGX_CHECK_LAUNCH();
       far_base = s.roff_far;
       near_base = s.roff_near;
     }
-    if (far_records > 0) {
-      k_tw_copy_raw<<<grid_for((int64_t)far_records * 32, 256, kNumSMs * 16), 256, 0, stream>>>(
-          s.far_keys, s.far_recs, (int64_t)far_records, far_base, total, s.far_pool, c.far,
-          far_raw, far_raw_cap, s.status);
-      YGX_CHECK_LAUNCH();
-    }
-    if (near_records > 0) {
-      k_tw_copy_raw<<<grid_for((int64_t)near_records * 32, 256, kNumSMs * 16), 256, 0, stream>>>(
-          s.near_keys, s.near_recs, (int64_t)near_records, near_base, L, s.near_pool, c.near_,
-          near_raw, near_raw_cap, s.status);
+    const int64_t records =
+        (int64_t)(far_records > near_records ? far_records : near_records);
+    if (records > 0) {
+      k_tw_copy_raw<<<dim3(grid_for(records * 32, 256, kNumSMs * 16), 2), 256, 0, stream>>>(
+          TwCopy{s.far_keys, s.far_recs, (int64_t)far_records, far_base, total, s.far_pool, c.far,
+                 far_raw, far_raw_cap},
+          TwCopy{s.near_keys, s.near_recs, (int64_t)near_records, near_base, L, s.near_pool,
+                 c.near_, near_raw, near_raw_cap},
+          s.status);
       YGX_CHECK_LAUNCH();
     }
     const RowTable far_rows{total, s.far_off_node, s.far_cnt, level32, far_raw,
@@ -1843,7 +1858,7 @@ int ygx_target_walk_lists(int64_t total, int64_t num_internal, const int64_t* ca
     }
   }
   if (max_nbr > 0 && neighbor_leaf_positions && leafpos32 && L > 0) {
-    k_tw_nbr_leaf_pos<<<grid_for(L * max_nbr, 256), 256, 0, stream>>>(
+    k_tw_nbr_leaf_pos<<<grid_for(L * 32, 256), 256, 0, stream>>>(
         s.near_off, s.near_cnt, L, neighbors, index_bits, leafpos32, max_nbr,
         neighbor_leaf_positions);
     YGX_CHECK_LAUNCH();
@@ -1856,7 +1871,7 @@ int ygx_target_walk_lists(int64_t total, int64_t num_internal, const int64_t* ca
 // sums_out (host, 2) = the two totals.  Synchronizes the stream.
 size_t ygx_target_pad_workspace_size(int64_t total, int64_t num_leaves) {
   const int64_t m = total > num_leaves ? total : num_leaves;
-  return sizeof(int64_t) * ygx::scan_scratch_elems(m > 0 ? m : 1) + 256;
+  return sizeof(int64_t) * (ygx::seg_scan_elems(m > 0 ? m : 1, 2) + 2) + 256;
 }
 
 int ygx_target_pad(int64_t total, int64_t num_leaves, const int32_t* far_rcap32,
@@ -1868,16 +1883,12 @@ int ygx_target_pad(int64_t total, int64_t num_leaves, const int32_t* far_rcap32,
       ws_bytes < ygx_target_pad_workspace_size(total, num_leaves))
     return YGX_ERR_ARG;
   if (reinterpret_cast<uintptr_t>(ws) % sizeof(int64_t)) return YGX_ERR_ARG;
-  int64_t* tmp = reinterpret_cast<int64_t*>(ws);
-  int rc = exclusive_scan<int32_t>(far_rcap32, total, pad_far, tmp, stream);
-  if (rc) return rc;
-  rc = exclusive_scan<int32_t>(near_rcap32, num_leaves, pad_near, tmp, stream);
+  int64_t* tmp = reinterpret_cast<int64_t*>(ws);  // the two totals, then the scans' scratch
+  const TwPad pad{far_rcap32, near_rcap32, total, num_leaves, pad_far, pad_near, tmp};
+  const int rc = seg_scan(pad, total, 2, tmp + 2, stream);
   if (rc) return rc;
   int64_t sums[2];
-  if (cudaMemcpyAsync(&sums[0], pad_far + total, sizeof(int64_t), cudaMemcpyDeviceToHost,
-                      stream) != cudaSuccess ||
-      cudaMemcpyAsync(&sums[1], pad_near + num_leaves, sizeof(int64_t), cudaMemcpyDeviceToHost,
-                      stream) != cudaSuccess ||
+  if (cudaMemcpyAsync(sums, tmp, sizeof(sums), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
       cudaStreamSynchronize(stream) != cudaSuccess)
     return YGX_ERR_CUDA;
   sums_out[0] = (uint64_t)sums[0];

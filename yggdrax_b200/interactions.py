@@ -555,7 +555,7 @@ def _target_walk(topology, d, total, ni, nl, num_levels, center, radius, max_ext
             L.ptr(near_rcap), st), "ygx_predict_caps")
         pad_far = torch.empty(total + 1, dtype=torch.int64, device=dev)
         pad_near = torch.empty(nl + 1, dtype=torch.int64, device=dev)
-        pws = L.workspace(lib.ygx_target_pad_workspace_size(total, nl), dev)
+        pws = L.workspace(lib.ygx_target_pad_workspace_size(total, nl), dev, zero=False)
         sums = np.zeros(2, np.uint64)
         L.check(lib.ygx_target_pad(total, nl, L.ptr(far_rcap), L.ptr(near_rcap), L.ptr(pad_far),
                                    L.ptr(pad_near), sums.ctypes.data, L.ptr(pws), pws.numel(), st),
@@ -577,7 +577,7 @@ def _target_walk(topology, d, total, ni, nl, num_levels, center, radius, max_ext
             pred = (L.ptr(far_rcap), L.ptr(near_rcap), L.ptr(pad_far), L.ptr(pad_near),
                     L.ptr(far_raw), L.ptr(near_raw))
         ws = L.workspace(lib.ygx_target_walk_workspace_size(total, nl, caps_np.ctypes.data, o),
-                         dev)
+                         dev, zero=False)
         stats = np.zeros(L.TSTAT_WORDS, np.uint64)
         needs = np.zeros(14, np.uint64)
         flags = np.zeros(1, np.uint32)
