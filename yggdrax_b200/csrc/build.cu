@@ -1,5 +1,6 @@
 // Tree build kernels (L1): reorder, leaf partitions (adaptive, fixed depth,
 // local aspect refinement), Karras LBVH topology and node levels.
+#include "genwalk.cuh"
 #include "scan.cuh"
 #include "karras.cuh"
 #include "sort.cuh"
@@ -285,146 +286,289 @@ __global__ void k_refine(const float* __restrict__ pos_sorted, const uint64_t* _
   }
 }
 
-__global__ void k_karras(const uint64_t* __restrict__ codes, const void* starts, const void* ends,
-                         int64_t L, int index_bits, void* left, void* right,
-                         uint8_t* __restrict__ lil, uint8_t* __restrict__ ril, void* ranges,
-                         int32_t* __restrict__ left32, int32_t* __restrict__ right32,
-                         int32_t* __restrict__ parent_claim) {
-  const int64_t ni = L - 1;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ni;
-       i += (int64_t)gridDim.x * blockDim.x)
-    karras_node(codes, starts, ends, L, i, index_bits, left, right, lil, ril, ranges, left32,
-                right32, parent_claim, 0);
-}
+// ---------------------------------------------------------------------------
+// Depths (_tree_impl.py:1272-1299, synchronous pointer doubling over a fixed
+// number of rounds).  A node whose parent chain ends has the chain's length,
+// so each thread climbs: neighbours share their ancestors, the chain is short
+// (63-bit codes without ties: at most 64 nodes) and its loads hit L1.  Longer
+// chains -- cycles among them, which tied codes can produce and whose "depth"
+// is 2^rounds -- make every CTA run the doubling itself.
+constexpr int kClimbMax = 128;
 
-__global__ void k_leaf_ranges(const void* starts, const void* ends, int64_t L, int index_bits,
-                              void* ranges, int32_t* __restrict__ left32,
-                              int32_t* __restrict__ right32) {
-  const int64_t ni = L - 1;
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < L;
-       j += (int64_t)gridDim.x * blockDim.x) {
-    store_idx(ranges, index_bits, 2 * (ni + j), load_idx(starts, index_bits, j));
-    store_idx(ranges, index_bits, 2 * (ni + j) + 1, load_idx(ends, index_bits, j) - 1);
-    left32[ni + j] = -1;
-    right32[ni + j] = -1;
+struct DepthArgs {
+  const int32_t* parent;  // -1 at roots
+  int64_t total;
+  int32_t rounds;
+  int32_t* depth;         // out
+  int32_t* root;          // out: where the chain ends
+  int32_t* sc2;           // the doubling's second buffers
+  int32_t* d2;
+  uint32_t* deep;         // zeroed: some chain is too long to climb
+  unsigned* arrived;      // zeroed: grid barrier
+  uint32_t spin_limit;
+};
+
+// Depth and chain end of every node, in a cooperative launch; false when the
+// barrier gave up.  The last barrier has passed on return.
+__device__ bool find_depths(const DepthArgs& a, unsigned* target) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  bool deep = false;
+  for (int64_t k = t0; k < a.total; k += stride) {
+    int32_t d = 0, v = (int32_t)k, p = a.parent[k];
+    while (p >= 0 && d < kClimbMax) {
+      v = p;
+      ++d;
+      p = a.parent[v];
+    }
+    deep |= p >= 0;
+    a.depth[k] = d;
+    a.root[k] = v;
   }
-}
-
-// Decode the claims into parent, and flag any internal node whose children
-// do not name it back (a malformed topology from tied codes).
-__global__ void k_parent_decode(const int32_t* __restrict__ claim, int64_t total, int64_t ni,
-                                int index_bits, void* parent, int32_t* __restrict__ parent32) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    int32_t c = claim[k];
-    int64_t p = c < 0 ? -1 : (c >= ni ? c - ni : c);
-    store_idx(parent, index_bits, k, p);
-    parent32[k] = (int32_t)p;
-  }
-}
-
-__global__ void k_check_wellformed(const int32_t* __restrict__ parent32,
-                                   const int32_t* __restrict__ left32,
-                                   const int32_t* __restrict__ right32, int64_t total, int64_t ni,
-                                   uint32_t* __restrict__ tree_flags) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    bool bad = (k == 0) ? parent32[0] != -1 : parent32[k] < 0;
-    if (k < ni) bad = bad || parent32[left32[k]] != (int32_t)k || parent32[right32[k]] != (int32_t)k;
-    if (bad) atomicOr(tree_flags, kFlagMalformed);
-  }
-}
-
-// _tree_impl.py:1272-1299: depth by synchronous pointer doubling.  Rounds
-// after the state stops changing are no-ops, so a round that sees the
-// previous round unchanged returns at once; `stop` records how many rounds
-// actually ran so the final state can be read from the right buffer.
-__global__ void k_depth_init(const int32_t* __restrict__ parent32, int64_t total,
-                             int32_t* __restrict__ sc, int32_t* __restrict__ d) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    int32_t p = parent32[k];
+  if (__syncthreads_or(deep) && threadIdx.x == 0) atomicOr(a.deep, 1u);
+  if (!gen_barrier(a.arrived, target, a.spin_limit)) return false;
+  if (__ldcg(a.deep) == 0) return true;
+  int32_t *sc = a.root, *d = a.depth, *sn = a.sc2, *dn = a.d2;
+  for (int64_t k = t0; k < a.total; k += stride) {
+    const int32_t p = a.parent[k];
     sc[k] = p < 0 ? (int32_t)k : p;
     d[k] = p < 0 ? 0 : 1;
   }
-}
-
-__global__ void k_depth_round(const int32_t* __restrict__ sc_in, const int32_t* __restrict__ d_in,
-                              int32_t* __restrict__ sc_out, int32_t* __restrict__ d_out,
-                              int64_t total, int round, uint32_t* __restrict__ changed,
-                              uint32_t* __restrict__ stop) {
-  if (round > 0 && ((volatile uint32_t*)changed)[round - 1] == 0) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicMin(stop, (uint32_t)round);
-    return;
-  }
-  bool any = false;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    int32_t s = sc_in[k];
-    int32_t nd = d_in[k] + d_in[s];
-    int32_t ns = sc_in[s];
-    sc_out[k] = ns;
-    d_out[k] = nd;
-    any |= (ns != s) || (nd != d_in[k]);
-  }
-  if (__syncthreads_or(any) && threadIdx.x == 0) atomicOr(&changed[round], 1u);
-}
-
-// Final node levels (from whichever buffer holds the last state), the level
-// histogram over 64 bins and the 16-bit sort keys for nodes_by_level.
-__global__ void k_depth_finish(const int32_t* __restrict__ sc0, const int32_t* __restrict__ d0,
-                               const int32_t* __restrict__ sc1, const int32_t* __restrict__ d1,
-                               int64_t total, const uint32_t* __restrict__ stop, uint32_t rounds,
-                               int index_bits,
-                               void* node_level, int32_t* __restrict__ level32,
-                               uint64_t* __restrict__ level_keys, uint32_t* __restrict__ level_hist,
-                               int32_t* __restrict__ max_level, uint32_t* __restrict__ tree_flags) {
-  const uint32_t r = *stop < rounds ? *stop : rounds;
-  const int32_t* sc = (r & 1) ? sc1 : sc0;
-  const int32_t* d = (r & 1) ? d1 : d0;
-  __shared__ uint32_t s_hist[64];
-  if (threadIdx.x < 64) s_hist[threadIdx.x] = 0;
-  __syncthreads();
-  int32_t mx = 0;
-  bool detached = false;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    int32_t lv = d[k];
-    store_idx(node_level, index_bits, k, lv);
-    level32[k] = lv;
-    level_keys[k] = (uint64_t)(uint32_t)lv;
-    if (lv >= 0 && lv < 64) atomicAdd(&s_hist[lv], 1u);
-    mx = lv > mx ? lv : mx;
-    detached |= sc[k] != 0;
-  }
-  __syncthreads();
-  if (threadIdx.x < 64 && s_hist[threadIdx.x]) atomicAdd(&level_hist[threadIdx.x], s_hist[threadIdx.x]);
-  atomicMax(max_level, mx);
-  if (detached) atomicOr(tree_flags, kFlagMalformed);
-}
-
-__global__ void k_level_tables(const uint32_t* __restrict__ level_hist,
-                               const int32_t* __restrict__ max_level, int index_bits,
-                               void* level_offsets, void* num_levels) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    int64_t acc = 0;
-    store_idx(level_offsets, index_bits, 0, 0);
-    for (int l = 0; l < 64; ++l) {
-      acc += level_hist[l];
-      store_idx(level_offsets, index_bits, l + 1, acc);
+  if (!gen_barrier(a.arrived, target, a.spin_limit)) return false;
+  for (int r = 0; r < a.rounds; ++r) {
+    for (int64_t k = t0; k < a.total; k += stride) {
+      const int32_t s = __ldcg(sc + k);
+      dn[k] = __ldcg(d + k) + __ldcg(d + s);
+      sn[k] = __ldcg(sc + s);
     }
-    int64_t nl = (int64_t)(*max_level) + 1;
-    nl = nl < 1 ? 1 : (nl > 64 ? 64 : nl);
-    store_idx(num_levels, index_bits, 0, nl);
+    int32_t* x = sc;
+    sc = sn;
+    sn = x;
+    x = d;
+    d = dn;
+    dn = x;
+    if (!gen_barrier(a.arrived, target, a.spin_limit)) return false;
   }
+  if (d != a.depth) {
+    for (int64_t k = t0; k < a.total; k += stride) {
+      a.depth[k] = d[k];
+      a.root[k] = sc[k];
+    }
+    if (!gen_barrier(a.arrived, target, a.spin_limit)) return false;
+  }
+  return true;
 }
 
-__global__ void k_u32_to_index(const uint32_t* __restrict__ in, int64_t n, int index_bits,
-                               void* out, int32_t* __restrict__ out32) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    store_idx(out, index_bits, k, in[k]);
-    if (out32) out32[k] = (int32_t)in[k];
+__global__ void __launch_bounds__(kGenThreads, 2) k_depths(const DepthArgs a,
+                                                          uint32_t* __restrict__ status) {
+  unsigned target = 0;
+  if (!find_depths(a, &target) && threadIdx.x == 0) raise_flag(status, kFlagTimeout);
+}
+
+// ---------------------------------------------------------------------------
+// The whole topology of one tree in one cooperative launch: Karras search,
+// parents, the well-formedness check, depths, and the level tables with
+// nodes_by_level (a stable counting sort by depth).  Each stage is a few
+// microseconds of work on small trees and was a launch of its own (31 of them:
+// 11 to 21 rounds of pointer doubling, a two-pass radix sort of the levels).
+// Kernel time, 4,000 particles in leaves of 8: 62 -> 21 us (and 70 us of the
+// step); 16,777,216 in leaves of 32 (1 M nodes): 290 -> 116 us.
+struct TopoArgs {
+  const uint64_t* codes;
+  const void *starts, *ends;
+  int64_t L;
+  int index_bits;
+  void *parent, *left, *right;
+  uint8_t *lil, *ril;
+  void *ranges, *node_level, *level_offsets, *nbl, *num_levels;
+  int32_t *parent32, *left32, *right32, *level32, *nbl32;
+  int32_t* claim;
+  uint32_t* hist;        // per bin, per CTA
+  int32_t* by_low;       // nodes by the low digit of their level (two-digit levels)
+  int32_t* max_level;    // zeroed
+  uint32_t* tree_flags;  // zeroed
+  uint32_t* tree_flags_out;
+  uint32_t* status;
+  DepthArgs depth;
+};
+
+constexpr int kLevelBins = 64;   // levels of a tree without tied codes
+constexpr int kDigitBins = 256;  // digits of longer levels, sorted as 16-bit keys
+
+// One stable counting pass over `bins` digits (level >> shift) & (bins - 1) of
+// the nodes src[0..total) (null: 0, 1, ...): emits every node with its place.
+// With `counts`, the digit totals (of 64) are returned there.
+template <typename Emit>
+__device__ bool level_pass(const TopoArgs& a, unsigned* target, const int32_t* src, int bins,
+                           int shift, uint32_t* counts, Emit emit) {
+  __shared__ uint32_t s_bin[kDigitBins];              // histogram, then next place
+  __shared__ uint16_t s_warp[kGenWarps][kDigitBins];  // a chunk's counts per warp
+  const int64_t total = a.depth.total;
+  const int64_t slice = gen_slice(total);
+  const int64_t lo = blockIdx.x * slice, hi = lo + slice < total ? lo + slice : total;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto digit = [&](int32_t v) {
+    return (int)(((uint32_t)__ldcg(a.level32 + v) >> shift) & (uint32_t)(bins - 1));
+  };
+  for (int b = threadIdx.x; b < bins; b += kGenThreads) s_bin[b] = 0;
+  __syncthreads();
+  for (int64_t i = lo + threadIdx.x; i < hi; i += kGenThreads)
+    atomicAdd(&s_bin[digit(src ? __ldcg(src + i) : (int32_t)i)], 1u);
+  __syncthreads();
+  for (int b = threadIdx.x; b < bins; b += kGenThreads)
+    a.hist[(int64_t)b * gridDim.x + blockIdx.x] = s_bin[b];
+  if (!gen_barrier(a.depth.arrived, target, a.depth.spin_limit)) return false;
+  // per bin: its total (kept in s_warp's space as 32-bit words) and what the
+  // CTAs before this one hold
+  __shared__ uint32_t s_total[kDigitBins];
+  for (int b = warp; b < bins; b += kGenWarps) {
+    uint32_t all = 0, before = 0;
+    for (int c = lane; c < (int)gridDim.x; c += 32) {
+      const uint32_t v = __ldcg(a.hist + (int64_t)b * gridDim.x + c);
+      all += v;
+      if (c < (int)blockIdx.x) before += v;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      all += __shfl_xor_sync(0xffffffffu, all, o);
+      before += __shfl_xor_sync(0xffffffffu, before, o);
+    }
+    if (lane == 0) {
+      s_total[b] = all;
+      s_bin[b] = before;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t run = 0;
+    for (int b = 0; b < bins; ++b) {
+      if (counts && b < kLevelBins) counts[b] = s_total[b];
+      s_bin[b] += run;
+      run += s_total[b];
+    }
+  }
+  __syncthreads();
+  for (int64_t c0 = lo; c0 < hi; c0 += kGenThreads) {
+    for (int b = threadIdx.x; b < kGenWarps * bins; b += kGenThreads)
+      s_warp[b / bins][b % bins] = 0;
+    __syncthreads();
+    const int64_t i = c0 + threadIdx.x;
+    const bool live = i < hi;
+    const int32_t v = live ? (src ? __ldcg(src + i) : (int32_t)i) : 0;
+    const int d = live ? digit(v) : bins;
+    const unsigned peers = __match_any_sync(0xffffffffu, d);
+    const int rank = __popc(peers & ((1u << lane) - 1u));
+    if (live && rank == 0) s_warp[warp][d] = (uint16_t)__popc(peers);
+    __syncthreads();
+    for (int b = threadIdx.x; b < bins; b += kGenThreads) {
+      uint32_t run = 0;  // counts of the warps before, and the chunk's total
+      for (int w = 0; w < kGenWarps; ++w) {
+        const uint32_t c = s_warp[w][b];
+        s_warp[w][b] = (uint16_t)run;
+        run += c;
+      }
+      s_total[b] = run;
+    }
+    __syncthreads();
+    if (live) emit((int64_t)s_bin[d] + s_warp[warp][d] + rank, v);
+    __syncthreads();
+    for (int b = threadIdx.x; b < bins; b += kGenThreads) s_bin[b] += s_total[b];
+    __syncthreads();
+  }
+  return true;
+}
+
+__device__ bool build_topology(const TopoArgs& a) {
+  const int64_t L = a.L, ni = L - 1, total = 2 * L - 1;
+  const int ib = a.index_bits;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned target = 0;
+  for (int64_t k = t0; k < total; k += stride) a.claim[k] = -1;
+  if (!gen_barrier(a.depth.arrived, &target, a.depth.spin_limit)) return false;
+  for (int64_t j = t0; j < L; j += stride) {
+    store_idx(a.ranges, ib, 2 * (ni + j), load_idx(a.starts, ib, j));
+    store_idx(a.ranges, ib, 2 * (ni + j) + 1, load_idx(a.ends, ib, j) - 1);
+    a.left32[ni + j] = -1;
+    a.right32[ni + j] = -1;
+    if (j < ni)
+      karras_node(a.codes, a.starts, a.ends, L, j, ib, a.left, a.right, a.lil, a.ril, a.ranges,
+                  a.left32, a.right32, a.claim, 0);
+  }
+  if (!gen_barrier(a.depth.arrived, &target, a.depth.spin_limit)) return false;
+  // the claims as parents
+  for (int64_t k = t0; k < total; k += stride) {
+    const int32_t c = __ldcg(a.claim + k);
+    const int64_t p = c < 0 ? -1 : (c >= ni ? c - ni : c);
+    store_idx(a.parent, ib, k, p);
+    a.parent32[k] = (int32_t)p;
+  }
+  if (!gen_barrier(a.depth.arrived, &target, a.depth.spin_limit)) return false;
+  // malformed (tied codes): a node whose children do not name it back, or a
+  // second root
+  bool bad = false;
+  for (int64_t k = t0; k < total; k += stride) {
+    bad |= (k == 0) ? a.parent32[0] != -1 : a.parent32[k] < 0;
+    if (k < ni)
+      bad |= a.parent32[__ldcg(a.left32 + k)] != (int32_t)k ||
+             a.parent32[__ldcg(a.right32 + k)] != (int32_t)k;
+  }
+  if (!find_depths(a.depth, &target)) return false;
+  int32_t mx = 0;
+  for (int64_t k = t0; k < total; k += stride) {
+    const int32_t lv = a.level32[k];
+    store_idx(a.node_level, ib, k, lv);
+    mx = lv > mx ? lv : mx;
+    bad |= a.depth.root[k] != 0;  // a detached node
+  }
+  if (bad) atomicOr(a.tree_flags, kFlagMalformed);
+  for (int o = 16; o > 0; o >>= 1) {
+    const int32_t w = __shfl_xor_sync(0xffffffffu, mx, o);
+    mx = w > mx ? w : mx;
+  }
+  if ((threadIdx.x & 31) == 0 && mx > 0) atomicMax(a.max_level, mx);
+  if (!gen_barrier(a.depth.arrived, &target, a.depth.spin_limit)) return false;
+  const int32_t deepest = __ldcg(a.max_level);
+  __shared__ uint32_t s_counts[kLevelBins];
+  auto place = [&](int64_t at, int32_t v) {
+    store_idx(a.nbl, ib, at, v);
+    a.nbl32[at] = v;
+  };
+  if (deepest < kLevelBins) {
+    if (!level_pass(a, &target, nullptr, kLevelBins, 0, s_counts, place)) return false;
+  } else {
+    // 16-bit levels by two digits; the counts of levels 0..63 are their own
+    if (threadIdx.x < kLevelBins) s_counts[threadIdx.x] = 0;
+    __syncthreads();
+    if (blockIdx.x == 0)
+      for (int64_t k = threadIdx.x; k < total; k += kGenThreads) {
+        const int32_t lv = __ldcg(a.level32 + k);
+        if (lv >= 0 && lv < kLevelBins) atomicAdd(&s_counts[lv], 1u);
+      }
+    if (!level_pass(a, &target, nullptr, kDigitBins, 0, nullptr,
+                    [&](int64_t at, int32_t v) { a.by_low[at] = v; }))
+      return false;
+    if (!gen_barrier(a.depth.arrived, &target, a.depth.spin_limit)) return false;
+    if (!level_pass(a, &target, a.by_low, kDigitBins, 8, nullptr, place)) return false;
+  }
+  __syncthreads();
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    int64_t acc = 0;
+    store_idx(a.level_offsets, ib, 0, 0);
+    for (int l = 0; l < kLevelBins; ++l) {
+      acc += s_counts[l];
+      store_idx(a.level_offsets, ib, l + 1, acc);
+    }
+    const int64_t nl = (int64_t)deepest + 1;
+    store_idx(a.num_levels, ib, 0, nl < 1 ? 1 : (nl > 64 ? 64 : nl));
+    if (a.tree_flags_out) *a.tree_flags_out = __ldcg(a.tree_flags);
+  }
+  return true;
+}
+
+__global__ void __launch_bounds__(kGenThreads, 2) k_topology(const TopoArgs a) {
+  if (!build_topology(a) && threadIdx.x == 0) {
+    raise_flag(a.status, kFlagTimeout);
+    if (a.tree_flags_out) raise_flag(a.tree_flags_out, kFlagTimeout);
   }
 }
 
@@ -579,34 +723,40 @@ __global__ void k_seg_check_wellformed(const int32_t* __restrict__ parent32,
 // Levels of the forest (pointer doubling ran over all sets at once), the
 // per-set level histograms and maxima, and (set, level) sort keys.  A node
 // whose root is not its set's node 0 marks its set malformed.
-__global__ void k_seg_depth_finish(const int32_t* __restrict__ sc0, const int32_t* __restrict__ d0,
-                                   const int32_t* __restrict__ sc1, const int32_t* __restrict__ d1,
-                                   int64_t total, const uint32_t* __restrict__ stop,
-                                   uint32_t rounds, const int32_t* __restrict__ node_seg,
+__global__ void k_seg_depth_finish(const int32_t* __restrict__ sc, const int32_t* __restrict__ d,
+                                   int64_t total, const int32_t* __restrict__ node_seg,
                                    const int64_t* __restrict__ leaf_off, int index_bits,
                                    void* node_level, int32_t* __restrict__ level32,
                                    uint64_t* __restrict__ level_keys,
                                    uint32_t* __restrict__ seg_hist,
                                    int32_t* __restrict__ seg_max, uint32_t* __restrict__ seg_flags,
                                    uint32_t* __restrict__ tree_flags) {
-  const uint32_t r = *stop < rounds ? *stop : rounds;
-  const int32_t* sc = (r & 1) ? sc1 : sc0;
-  const int32_t* d = (r & 1) ? d1 : d0;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t sg = node_seg[k];
-    const int64_t NO = 2 * leaf_off[sg] - sg;
-    const int32_t lv = d[k];
-    store_idx(node_level, index_bits, k, lv);
-    level32[k] = lv;
-    const uint32_t klv = lv < 0 ? 0u : (lv > 0xFFFF ? 0xFFFFu : (uint32_t)lv);
-    level_keys[k] = ((uint64_t)(uint32_t)sg << 16) | klv;
-    if (lv >= 0 && lv < 64) atomicAdd(&seg_hist[(int64_t)sg * 64 + lv], 1u);
-    atomicMax(&seg_max[sg], lv);
-    if (sc[k] != (int32_t)NO) {
-      atomicOr(&seg_flags[sg], kFlagMalformed);
-      atomicOr(tree_flags, kFlagMalformed);
+  const int lane = threadIdx.x & 31;
+  for (int64_t k0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; k0 < total;
+       k0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t k = k0 + lane;
+    const bool live = k < total;
+    const int32_t sg = live ? node_seg[k] : -1, lv = live ? d[k] : -1;
+    if (live) {
+      store_idx(node_level, index_bits, k, lv);
+      level32[k] = lv;
+      const uint32_t klv = lv < 0 ? 0u : (lv > 0xFFFF ? 0xFFFFu : (uint32_t)lv);
+      level_keys[k] = ((uint64_t)(uint32_t)sg << 16) | klv;
+      if (sc[k] != (int32_t)(2 * leaf_off[sg] - sg)) {
+        atomicOr(&seg_flags[sg], kFlagMalformed);
+        atomicOr(tree_flags, kFlagMalformed);
+      }
     }
+    // a warp's nodes lie in one set mostly and share a few levels: one atomic
+    // per distinct (set, level), one maximum per warp and set (one of each per
+    // node: 192 us for 673,000 nodes, 23 us so)
+    const unsigned peers =
+        __match_any_sync(0xffffffffu, ((unsigned long long)(uint32_t)sg << 32) | (uint32_t)lv);
+    if (live && lane == __ffs(peers) - 1 && lv >= 0 && lv < 64)
+      atomicAdd(&seg_hist[(int64_t)sg * 64 + lv], (uint32_t)__popc(peers));
+    const unsigned same = __match_any_sync(0xffffffffu, sg);
+    const int32_t mx = __reduce_max_sync(same, lv);
+    if (live && lane == __ffs(same) - 1) atomicMax(&seg_max[sg], mx);
   }
 }
 
@@ -652,14 +802,10 @@ struct TopoScratch {
   int32_t* parent_claim;
   int32_t* sc[2];
   int32_t* d[2];
-  uint32_t* changed;
-  uint32_t* stop;
-  uint32_t* level_hist;
+  uint32_t* deep;
+  unsigned* arrived;
+  uint32_t* hist;
   int32_t* max_level;
-  uint64_t* level_keys;
-  uint64_t* level_keys_sorted;
-  uint32_t* nbl_u32;
-  SortScratch sort;
 };
 
 static TopoScratch carve_topo(Arena& a, int64_t L) {
@@ -667,17 +813,32 @@ static TopoScratch carve_topo(Arena& a, int64_t L) {
   TopoScratch s;
   s.status = a.take<uint32_t>(64);
   s.tree_flags = a.take<uint32_t>(64);
-  s.changed = a.take<uint32_t>(128);
-  s.stop = a.take<uint32_t>(64);
-  s.level_hist = a.take<uint32_t>(64);
+  s.deep = a.take<uint32_t>(64);
+  s.arrived = a.take<unsigned>(64);
   s.max_level = a.take<int32_t>(64);
+  s.hist = a.take<uint32_t>((size_t)kDigitBins * kGenMaxBlocks);
   s.parent_claim = a.take<int32_t>(total);
   for (int b = 0; b < 2; ++b) { s.sc[b] = a.take<int32_t>(total); s.d[b] = a.take<int32_t>(total); }
-  s.level_keys = a.take<uint64_t>(total);
-  s.level_keys_sorted = a.take<uint64_t>(total);
-  s.nbl_u32 = a.take<uint32_t>(total);
-  s.sort = carve_sort_scratch(a, total, 2);
   return s;
+}
+
+// A cooperative launch over n items with as many CTAs as they fill (a small
+// tree's barriers are cheap), at most what the device holds at once.
+template <typename Kernel, typename Args, typename... Rest>
+static int launch_cooperative(Kernel kernel, Args args, int64_t n, cudaStream_t stream,
+                              Rest... rest) {
+  int grid = gen_grid(kernel);
+  const int64_t want = (n + kGenThreads - 1) / kGenThreads;
+  if (want < grid) grid = (int)want;
+  void* params[] = {&args, &rest...};
+  if (grid < 1 || cudaLaunchCooperativeKernel((const void*)kernel, dim3((unsigned)grid),
+                                              dim3(kGenThreads), params, 0,
+                                              stream) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return YGX_ERR_CUDA;
+  }
+  YGX_CHECK_LAUNCH();
+  return YGX_OK;
 }
 
 }  // namespace ygx
@@ -829,58 +990,45 @@ int ygx_build_topology(const uint64_t* leaf_codes, const void* leaf_starts, cons
   if (ws_bytes < ygx_topology_workspace_size(L)) return YGX_ERR_ARG;
   ygx::Arena a{(char*)ws, 0, ws_bytes};
   ygx::TopoScratch s = ygx::carve_topo(a, L);
-  const int64_t total = 2 * L - 1, ni = L - 1;
-  // flags, changed, stop, hist, max_level are contiguous: one memset.
+  const int64_t total = 2 * L - 1;
+  // flags, barrier and maximum are contiguous: one memset
   if (cudaMemsetAsync(s.tree_flags, 0, (char*)(s.max_level + 64) - (char*)s.tree_flags, stream) !=
       cudaSuccess)
     return YGX_ERR_CUDA;
-  if (cudaMemsetAsync(s.stop, 0xFF, 64 * sizeof(uint32_t), stream) != cudaSuccess) return YGX_ERR_CUDA;
-  if (cudaMemsetAsync(s.parent_claim, 0xFF, total * sizeof(int32_t), stream) != cudaSuccess)
-    return YGX_ERR_CUDA;
-  ygx::k_karras<<<ygx::grid_for(L, 256), 256, 0, stream>>>(
-      leaf_codes, leaf_starts, leaf_ends, L, index_bits, left, right, left_is_leaf, right_is_leaf,
-      node_ranges, left32, right32, s.parent_claim);
-  YGX_CHECK_LAUNCH();
-  ygx::k_leaf_ranges<<<ygx::grid_for(L, 256), 256, 0, stream>>>(leaf_starts, leaf_ends, L,
-                                                                index_bits, node_ranges, left32,
-                                                                right32);
-  YGX_CHECK_LAUNCH();
-  ygx::k_parent_decode<<<ygx::grid_for(total, 256), 256, 0, stream>>>(s.parent_claim, total, ni,
-                                                                      index_bits, parent, parent32);
-  YGX_CHECK_LAUNCH();
-  ygx::k_check_wellformed<<<ygx::grid_for(total, 256), 256, 0, stream>>>(
-      parent32, left32, right32, total, ni, s.tree_flags);
-  YGX_CHECK_LAUNCH();
-  // Levels by pointer doubling: bit_length(total) + 1 rounds.
-  int bl = 0;
+  int bl = 0;  // the reference's doubling rounds: bit_length(total) + 1
   while (((int64_t)1 << bl) <= total) ++bl;
-  const int rounds = bl + 1 > 1 ? bl + 1 : 1;
-  ygx::k_depth_init<<<ygx::grid_for(total, 256), 256, 0, stream>>>(parent32, total, s.sc[0], s.d[0]);
-  YGX_CHECK_LAUNCH();
-  for (int r = 0; r < rounds; ++r) {
-    ygx::k_depth_round<<<ygx::grid_for(total, 256), 256, 0, stream>>>(
-        s.sc[r & 1], s.d[r & 1], s.sc[(r + 1) & 1], s.d[(r + 1) & 1], total, r, s.changed, s.stop);
-    YGX_CHECK_LAUNCH();
-  }
-  ygx::k_depth_finish<<<ygx::grid_for(total, 256), 256, 0, stream>>>(
-      s.sc[0], s.d[0], s.sc[1], s.d[1], total, s.stop, (uint32_t)rounds, index_bits, node_level,
-      level32, s.level_keys, s.level_hist, s.max_level, s.tree_flags);
-  YGX_CHECK_LAUNCH();
-  ygx::k_level_tables<<<1, 32, 0, stream>>>(s.level_hist, s.max_level, index_bits, level_offsets,
-                                            num_levels);
-  YGX_CHECK_LAUNCH();
-  // nodes_by_level: stable argsort of node_level (levels < 2^16).
-  int rc = ygx::onesweep_sort(s.level_keys, nullptr, total, 0, 16, s.level_keys_sorted, s.nbl_u32,
-                              s.sort, false, s.status, stream);
-  if (rc) return rc;
-  ygx::k_u32_to_index<<<ygx::grid_for(total, 256), 256, 0, stream>>>(s.nbl_u32, total, index_bits,
-                                                                     nodes_by_level, nbl32);
-  YGX_CHECK_LAUNCH();
-  if (tree_flags_out &&
-      cudaMemcpyAsync(tree_flags_out, s.tree_flags, sizeof(uint32_t), cudaMemcpyDeviceToDevice,
-                      stream) != cudaSuccess)
-    return YGX_ERR_CUDA;
-  return YGX_OK;
+  ygx::TopoArgs t;
+  t.codes = leaf_codes;
+  t.starts = leaf_starts;
+  t.ends = leaf_ends;
+  t.L = L;
+  t.index_bits = index_bits;
+  t.parent = parent;
+  t.left = left;
+  t.right = right;
+  t.lil = left_is_leaf;
+  t.ril = right_is_leaf;
+  t.ranges = node_ranges;
+  t.node_level = node_level;
+  t.level_offsets = level_offsets;
+  t.nbl = nodes_by_level;
+  t.num_levels = num_levels;
+  t.parent32 = parent32;
+  t.left32 = left32;
+  t.right32 = right32;
+  t.level32 = level32;
+  t.nbl32 = nbl32;
+  t.claim = s.parent_claim;
+  t.hist = s.hist;
+  t.by_low = s.parent_claim;  // free once the parents are known
+  t.max_level = s.max_level;
+  t.tree_flags = s.tree_flags;
+  t.tree_flags_out = tree_flags_out;
+  t.status = s.status;
+  t.depth = ygx::DepthArgs{parent32, total,  bl + 1,    level32,
+                           s.sc[0],  s.sc[1], s.d[1],   s.deep,
+                           s.arrived, (uint32_t)ygx::g_tune.spin_limit};
+  return ygx::launch_cooperative(ygx::k_topology, t, total, stream);
 }
 
 
@@ -946,35 +1094,40 @@ int ygx_batch_leaves(const uint64_t* codes_sorted, const int64_t* offsets, const
   return YGX_OK;
 }
 
-static ygx::TopoScratch carve_seg_topo(ygx::Arena& a, int64_t total, int64_t S,
-                                       uint32_t** seg_hist, int32_t** seg_max,
-                                       int32_t** node_seg_tmp) {
-  ygx::TopoScratch s;
+struct SegTopoScratch {
+  uint32_t *status, *tree_flags, *deep;
+  unsigned* arrived;
+  uint32_t* seg_hist;
+  int32_t* seg_max;
+  int32_t* parent_claim;
+  int32_t* sc[2];
+  int32_t* d[2];
+  uint64_t *level_keys, *level_keys_sorted;
+  uint32_t* nbl_u32;
+  ygx::SortScratch sort;
+};
+
+static SegTopoScratch carve_seg_topo(ygx::Arena& a, int64_t total, int64_t S) {
+  SegTopoScratch s;
   s.status = a.take<uint32_t>(64);
   s.tree_flags = a.take<uint32_t>(64);
-  s.changed = a.take<uint32_t>(128);
-  s.stop = a.take<uint32_t>(64);
-  s.level_hist = a.take<uint32_t>(64);
-  s.max_level = a.take<int32_t>(64);
-  *seg_hist = a.take<uint32_t>((size_t)S * 64);
-  *seg_max = a.take<int32_t>(S);
+  s.deep = a.take<uint32_t>(64);
+  s.arrived = a.take<unsigned>(64);
+  s.seg_hist = a.take<uint32_t>((size_t)S * 64);
+  s.seg_max = a.take<int32_t>(S);
   s.parent_claim = a.take<int32_t>(total);
   for (int b = 0; b < 2; ++b) { s.sc[b] = a.take<int32_t>(total); s.d[b] = a.take<int32_t>(total); }
   s.level_keys = a.take<uint64_t>(total);
   s.level_keys_sorted = a.take<uint64_t>(total);
   s.nbl_u32 = a.take<uint32_t>(total);
-  *node_seg_tmp = nullptr;
   s.sort = ygx::carve_sort_scratch(a, total, 4);
   return s;
 }
 
 size_t ygx_batch_topology_workspace_size(int64_t total_leaves, int64_t S) {
   ygx::Arena a{nullptr, 0, 0};
-  uint32_t* h;
-  int32_t* m;
-  int32_t* t;
   const int64_t total = total_leaves > S ? 2 * total_leaves - S : 1;
-  carve_seg_topo(a, total, S > 0 ? S : 1, &h, &m, &t);
+  carve_seg_topo(a, total, S > 0 ? S : 1);
   return a.used + 256;
 }
 
@@ -1005,14 +1158,10 @@ int ygx_batch_build_topology(const uint64_t* leaf_codes, const void* leaf_starts
   if (total >= (int64_t)INT32_MAX / 2) return YGX_ERR_ARG;
   if (ws_bytes < ygx_batch_topology_workspace_size(total_leaves, S)) return YGX_ERR_ARG;
   ygx::Arena a{(char*)ws, 0, ws_bytes};
-  uint32_t* seg_hist;
-  int32_t* seg_max;
-  int32_t* unused;
-  ygx::TopoScratch s = carve_seg_topo(a, total, S, &seg_hist, &seg_max, &unused);
-  // flags, changed, stop, hist, max_level, seg_hist, seg_max are contiguous
-  if (cudaMemsetAsync(s.tree_flags, 0, (char*)(seg_max + S) - (char*)s.tree_flags, stream) !=
+  SegTopoScratch s = carve_seg_topo(a, total, S);
+  // flags, barrier, histograms and maxima are contiguous
+  if (cudaMemsetAsync(s.tree_flags, 0, (char*)(s.seg_max + S) - (char*)s.tree_flags, stream) !=
           cudaSuccess ||
-      cudaMemsetAsync(s.stop, 0xFF, 64 * sizeof(uint32_t), stream) != cudaSuccess ||
       cudaMemsetAsync(s.parent_claim, 0xFF, total * sizeof(int32_t), stream) != cudaSuccess ||
       cudaMemsetAsync(seg_flags, 0, S * sizeof(uint32_t), stream) != cudaSuccess)
     return YGX_ERR_CUDA;
@@ -1029,24 +1178,20 @@ int ygx_batch_build_topology(const uint64_t* leaf_codes, const void* leaf_starts
   YGX_CHECK_LAUNCH();
   int bl = 0;
   while (((int64_t)1 << bl) <= total) ++bl;
-  const int rounds = bl + 1;
-  ygx::k_depth_init<<<ygx::grid_for(total, 256), 256, 0, stream>>>(parent32, total, s.sc[0], s.d[0]);
-  YGX_CHECK_LAUNCH();
-  for (int r = 0; r < rounds; ++r) {
-    ygx::k_depth_round<<<ygx::grid_for(total, 256), 256, 0, stream>>>(
-        s.sc[r & 1], s.d[r & 1], s.sc[(r + 1) & 1], s.d[(r + 1) & 1], total, r, s.changed, s.stop);
-    YGX_CHECK_LAUNCH();
-  }
+  ygx::DepthArgs depth{parent32, total,   bl + 1, s.d[0],    s.sc[0],
+                       s.sc[1],  s.d[1],  s.deep, s.arrived, (uint32_t)ygx::g_tune.spin_limit};
+  int rc = ygx::launch_cooperative(ygx::k_depths, depth, total, stream, s.tree_flags);
+  if (rc) return rc;
   ygx::k_seg_depth_finish<<<ygx::grid_for(total, 256), 256, 0, stream>>>(
-      s.sc[0], s.d[0], s.sc[1], s.d[1], total, s.stop, (uint32_t)rounds, node_seg32, leaf_off,
-      index_bits, node_level, level32, s.level_keys, seg_hist, seg_max, seg_flags, s.tree_flags);
+      s.sc[0], s.d[0], total, node_seg32, leaf_off, index_bits, node_level, level32, s.level_keys,
+      s.seg_hist, s.seg_max, seg_flags, s.tree_flags);
   YGX_CHECK_LAUNCH();
   ygx::k_seg_level_tables<<<ygx::grid_for(S, 128), 128, 0, stream>>>(
-      seg_hist, seg_max, leaf_off, S, index_bits, level_offsets, num_levels);
+      s.seg_hist, s.seg_max, leaf_off, S, index_bits, level_offsets, num_levels);
   YGX_CHECK_LAUNCH();
   // nodes_by_level: stable sort by (set, level); sets < 2^16, levels < 2^16
-  int rc = ygx::onesweep_sort(s.level_keys, nullptr, total, 0, 32, s.level_keys_sorted, s.nbl_u32,
-                              s.sort, false, s.status, stream);
+  rc = ygx::onesweep_sort(s.level_keys, nullptr, total, 0, 32, s.level_keys_sorted, s.nbl_u32,
+                          s.sort, false, s.status, stream);
   if (rc) return rc;
   ygx::k_seg_nbl<<<ygx::grid_for(total, 256), 256, 0, stream>>>(s.nbl_u32, node_seg32, leaf_off,
                                                                 total, index_bits,

@@ -38,7 +38,8 @@ __device__ __forceinline__ void karras_node(const uint64_t* __restrict__ codes,
     if (i == 0 || d == 0) d = 1;
     const int64_t dmin = kdelta(codes, L, i, i - d, ci);
     int64_t span = 0;
-    for (int k = 30; k >= 0; --k) {
+    // (a step of more than L - 1 is out of range: left out)
+    for (int k = 63 - clz64((uint64_t)L); k >= 0; --k) {
       int64_t step = (int64_t)1 << k;
       int64_t cand = i + (span + step) * d;
       if (cand >= 0 && cand < L && kdelta(codes, L, i, cand, ci) > dmin) span += step;
@@ -50,7 +51,7 @@ __device__ __forceinline__ void karras_node(const uint64_t* __restrict__ codes,
     const uint64_t fc = codes[first];
     const int64_t cp = lcp_codes(fc, codes[last]);
     int64_t split = first;
-    for (int k = 30; k >= 0; --k) {
+    for (int k = last > first ? 63 - clz64((uint64_t)(last - first)) : -1; k >= 0; --k) {
       int64_t mid = split + ((int64_t)1 << k);
       if (mid < last && lcp_codes(fc, codes[mid]) > cp) split = mid;
     }

@@ -461,6 +461,8 @@ def _build(positions, masses, bounds, *, build_mode: str, leaf_size: int = 8,
     # one read-back for the flags and the level count
     hv = torch.cat([topo._dev.tree_flags.to(torch.int64).reshape(1),
                     topo.num_levels.to(torch.int64).reshape(1)]).cpu()
+    if int(hv[0]) & L.FLAG_TIMEOUT:
+        raise L.YgxError("ygx_build_topology: a device-side wait gave up")
     topo._host = HostTopologyInfo(malformed=bool(int(hv[0]) & L.FLAG_MALFORMED),
                                   num_levels=int(hv[1]), use_morton=bool(use_morton))
     return topo, pos_sorted, mass_sorted, inv
