@@ -450,6 +450,15 @@ int ygx_node_order_far_rows(int64_t total, const void* far_counts, const void* n
 int ygx_flag_compact(const void* idx, int64_t n_idx, int64_t M, int index_bits,
                      int32_t* rank_out, void* cells_out, int64_t* count_out, void* ws,
                      size_t ws_bytes, cudaStream_t stream);
+/* The leaf tables of a traversal (_resolve_leaf_ordering,
+ * _interactions_impl.py:1071-1103): native (device, num_leaves = total -
+ * num_internal entries, or null for the identity) lists the leaves in native
+ * order.  leaf_indices[j] = node of native leaf j, particle_order[j] = node of
+ * leaf j, to_native = inverse of native (index dtype), leafpos32[node] =
+ * native position of a leaf, -1 on internal nodes (total entries). */
+int ygx_leaf_order(const uint32_t* native, int64_t total, int64_t num_internal, int index_bits,
+                   void* leaf_indices, void* particle_order, void* to_native, int32_t* leafpos32,
+                   cudaStream_t stream);
 /* out[j * width + k] = lookup[values[offsets[j] + k]] for k < counts[j], else
  * -1 (rows x width): the dense neighbor_leaf_positions table
  * (_interactions_impl.py:3658-3688).  lookup is int32 over lookup_n values. */

@@ -112,6 +112,7 @@ _SIGS = {
     "ygx_counts_to_offsets": (I32, [P, I64, I32, P, P, SZ, P]),
     "ygx_node_order_far_rows": (I32, [I64, P, P, P, I32, P, P, P, P, SZ, P]),
     "ygx_flag_compact": (I32, [P, I64, I64, I32, P, P, P, P, SZ, P]),
+    "ygx_leaf_order": (I32, [P, I64, I64, I32, P, P, P, P, P]),
     "ygx_dense_row_table": (I32, [P, P, I64, P, P, I64, I32, I64, P, P]),
     "ygx_gather_index": (I32, [P, I64, P, I64, I32, P, P, SZ, P]),
     "ygx_scatter_positions": (I32, [P, I32, I64, I64, P, I32, P, SZ, P]),
@@ -182,15 +183,15 @@ def exported_symbols() -> list:
     return sorted(_SIGS)
 
 
-def ptr(t: Optional[torch.Tensor]):
-    """Device pointer of a tensor (None -> NULL)."""
+def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
+    """Device pointer of a tensor (None -> NULL), as ctypes converts it."""
     if t is None:
         return None
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def stream_handle(device: torch.device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    return torch.cuda.current_stream(device).cuda_stream
 
 
 def check(rc: int, what: str) -> None:

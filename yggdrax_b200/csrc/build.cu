@@ -568,7 +568,7 @@ __device__ bool build_topology(const TopoArgs& a) {
 __global__ void __launch_bounds__(kGenThreads, 2) k_topology(const TopoArgs a) {
   if (!build_topology(a) && threadIdx.x == 0) {
     raise_flag(a.status, kFlagTimeout);
-    if (a.tree_flags_out) raise_flag(a.tree_flags_out, kFlagTimeout);
+    if (a.tree_flags_out) atomicExch(a.tree_flags_out, kFlagTimeout);
   }
 }
 

@@ -27,6 +27,27 @@ __global__ void k_store_offsets(const int64_t* __restrict__ off, int64_t n, int 
     store_idx(out, index_bits, i, off[i]);
 }
 
+// Native leaf order (native: a permutation of the leaves, or null for the
+// identity) as the four tables the lists carry.  Eight small tensor operations
+// took 100 us of host time in every traversal; this is one launch.
+__global__ void k_leaf_order(const uint32_t* __restrict__ native, int64_t total, int64_t ni,
+                             int index_bits, void* leaf_indices, void* particle_order,
+                             void* to_native, int32_t* __restrict__ leafpos) {
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total;
+       k += (int64_t)gridDim.x * blockDim.x) {
+    if (k < ni) {
+      leafpos[k] = -1;
+      continue;
+    }
+    const int64_t j = k - ni, v = native ? (int64_t)native[j] : j;
+    if (v >= total - ni) continue;
+    store_idx(particle_order, index_bits, j, k);
+    store_idx(leaf_indices, index_bits, j, ni + v);
+    store_idx(to_native, index_bits, v, j);
+    leafpos[ni + v] = (int32_t)j;
+  }
+}
+
 // One warp per node: its row, read at its level-major start, written at its
 // node-order start; targets = the node.
 __global__ void __launch_bounds__(256)
@@ -218,6 +239,19 @@ int ygx_flag_compact(const void* idx, int64_t n_idx, int64_t M, int index_bits,
       cudaStreamSynchronize(stream) != cudaSuccess)
     return YGX_ERR_CUDA;
   return flags ? YGX_ERR_ARG : YGX_OK;
+}
+
+int ygx_leaf_order(const uint32_t* native, int64_t total, int64_t num_internal, int index_bits,
+                   void* leaf_indices, void* particle_order, void* to_native, int32_t* leafpos32,
+                   cudaStream_t stream) {
+  if (total < 1 || total > INT32_MAX || num_internal < 0 || num_internal >= total ||
+      !leaf_indices || !particle_order || !to_native || !leafpos32 ||
+      (index_bits != 32 && index_bits != 64))
+    return YGX_ERR_ARG;
+  ygx::k_leaf_order<<<ygx::grid_for(total, 256), 256, 0, stream>>>(
+      native, total, num_internal, index_bits, leaf_indices, particle_order, to_native, leafpos32);
+  YGX_CHECK_LAUNCH();
+  return YGX_OK;
 }
 
 int ygx_dense_row_table(const void* offsets, const void* counts, int64_t rows, const void* values,

@@ -655,7 +655,11 @@ int ygx_encode_sort(const float* positions, int64_t n, const float* bounds_in, f
   // the 8-bit sort's digit histograms come out of the encode; the 11-bit
   // sort counts its own
   const int passes = ygx::sort_uses_wide(0, 63) ? 0 : ygx::sort_passes(0, 63);
-  if (ygx::sort_scratch_reset(l.sort, n, passes, stream) != cudaSuccess) return YGX_ERR_CUDA;
+  // status, partial boxes, arrival counters and the sort's tables lie one
+  // behind the other: one memset
+  if (cudaMemsetAsync(l.status, 0, (size_t)((char*)(l.sort.counters + 64) - (char*)l.status),
+                      stream) != cudaSuccess)
+    return YGX_ERR_CUDA;
   bool fused = false;
   if (!bounds_in) {
     // one cooperative launch: bounds, codes and histograms (see k_bbox_encode)
@@ -663,8 +667,6 @@ int ygx_encode_sort(const float* positions, int64_t n, const float* bounds_in, f
     if (grid > 0) {
       const int64_t want = ((n + 3) / 4 + ygx::kEncodeThreads - 1) / ygx::kEncodeThreads;
       if (want < grid) grid = want > 0 ? (int)want : 1;
-      if (cudaMemsetAsync(l.arrivals, 0, 2 * sizeof(unsigned), stream) != cudaSuccess)
-        return YGX_ERR_CUDA;
       const float* p_ = positions;
       int64_t n_ = n;
       float* part_ = l.partials;

@@ -59,7 +59,7 @@ def compute_tree_geometry(tree, positions_sorted: torch.Tensor, *,
     half = torch.empty((total, 3), dtype=torch.float32, device=dev)
     radius = torch.empty(total, dtype=torch.float32, device=dev)
     max_extent = torch.empty(total, dtype=torch.float32, device=dev)
-    ws = L.workspace(lib.ygx_geometry_workspace_size(total), dev)
+    ws = L.workspace(lib.ygx_geometry_workspace_size(total), dev, zero=False)
     L.check(lib.ygx_tree_geometry(
         L.ptr(topology.node_ranges), total, INDEX_BITS, L.ptr(d.parent32), L.ptr(d.left32),
         L.ptr(d.right32), L.ptr(d.level32), L.ptr(d.tree_flags), L.ptr(pos),

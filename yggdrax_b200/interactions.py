@@ -304,9 +304,9 @@ def _leaf_ordering(topology, total: int, ni: int, dev):
     """_resolve_leaf_ordering (:1071-1103): native leaf order (stable order
     of radix_leaf_to_oct for octrees), leaf positions, inverse map."""
     nl = total - ni
-    po = torch.arange(ni, total, dtype=INDEX_DTYPE, device=dev)
+    lib = L.lib()
+    native = None
     if hasattr(topology, "radix_leaf_to_oct"):
-        lib = L.lib()
         keys = topology.radix_leaf_to_oct.to(torch.int64).contiguous().view(torch.uint64)
         kout = torch.empty_like(keys)
         native = torch.empty(nl, dtype=torch.int32, device=dev)
@@ -314,14 +314,12 @@ def _leaf_ordering(topology, total: int, ni: int, dev):
         L.check(lib.ygx_sort_pairs(L.ptr(keys), None, nl, 0, 32, L.ptr(kout), L.ptr(native),
                                    L.ptr(ws), ws.numel(), L.stream_handle(dev)),
                 "ygx_sort_pairs")
-        native = native.to(torch.int64)
-    else:
-        native = torch.arange(nl, dtype=torch.int64, device=dev)
-    leaf_indices = po[native]
-    po_to_native = torch.empty(nl, dtype=INDEX_DTYPE, device=dev)
-    po_to_native[native] = torch.arange(nl, dtype=INDEX_DTYPE, device=dev)
-    leafpos32 = torch.full((total,), -1, dtype=torch.int32, device=dev)
-    leafpos32[leaf_indices.long()] = torch.arange(nl, dtype=torch.int32, device=dev)
+    leaf_indices, po, po_to_native = (torch.empty(nl, dtype=INDEX_DTYPE, device=dev)
+                                      for _ in range(3))
+    leafpos32 = torch.empty(total, dtype=torch.int32, device=dev)
+    L.check(lib.ygx_leaf_order(L.ptr(native), total, ni, INDEX_BITS, L.ptr(leaf_indices),
+                               L.ptr(po), L.ptr(po_to_native), L.ptr(leafpos32),
+                               L.stream_handle(dev)), "ygx_leaf_order")
     return leaf_indices, leafpos32, po, po_to_native
 
 

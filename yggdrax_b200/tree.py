@@ -295,7 +295,7 @@ def _encode_sort(pos, n, bounds_in, dev, st):
     bounds_dev = torch.empty(6, dtype=torch.float32, device=dev)
     codes = torch.empty(n, dtype=torch.uint64, device=dev)
     order = torch.empty(n, dtype=torch.int32, device=dev)
-    ws = _ws(lib.ygx_encode_sort_workspace_size(n), dev)
+    ws = L.workspace(lib.ygx_encode_sort_workspace_size(n), dev, zero=False)
     L.check(lib.ygx_encode_sort(L.ptr(pos), n, L.ptr(bounds_in), L.ptr(bounds_dev), L.ptr(codes),
                                 L.ptr(order), L.ptr(ws), ws.numel(), st), "ygx_encode_sort")
     return bounds_dev, codes, order, ws
@@ -397,7 +397,7 @@ def _build(positions, masses, bounds, *, build_mode: str, leaf_size: int = 8,
         raise ValueError(f"Unsupported build_mode '{build_mode}'")
 
     Lf = int(starts.shape[0])
-    bmin, bmax = bounds_dev[:3].clone(), bounds_dev[3:].clone()
+    bmin, bmax = bounds_dev.clone().view(2, 3).unbind(0)
     if Lf == 1:
         # _tree_impl.py:1052-1110
         level_offsets = torch.zeros(MAX_TREE_LEVELS + 1, dtype=idt, device=dev)
@@ -434,12 +434,13 @@ def _build(positions, masses, bounds, *, build_mode: str, leaf_size: int = 8,
         node_level = torch.empty(total, dtype=idt, device=dev)
         level_offsets = torch.empty(MAX_TREE_LEVELS + 1, dtype=idt, device=dev)
         nbl = torch.empty(total, dtype=idt, device=dev)
-        num_levels = torch.empty((), dtype=idt, device=dev)
+        # the level count and, behind it, the flags word: read back together
+        tail = torch.empty(2, dtype=idt, device=dev)
+        num_levels, flags = tail[0], tail[1:].view(torch.int32)[:1]
         i32 = dict(dtype=torch.int32, device=dev)
         parent32, left32, right32 = (torch.empty(total, **i32) for _ in range(3))
         level32, nbl32 = torch.empty(total, **i32), torch.empty(total, **i32)
-        flags = torch.zeros(1, **i32)
-        wst = _ws(lib.ygx_topology_workspace_size(Lf), dev)
+        wst = L.workspace(lib.ygx_topology_workspace_size(Lf), dev, zero=False)
         L.check(lib.ygx_build_topology(
             L.ptr(lcodes), L.ptr(starts), L.ptr(ends), Lf, ib, L.ptr(parent), L.ptr(left),
             L.ptr(right), L.ptr(lil), L.ptr(ril), L.ptr(ranges), L.ptr(node_level),
@@ -458,13 +459,14 @@ def _build(positions, masses, bounds, *, build_mode: str, leaf_size: int = 8,
                                    level32=level32, nbl32=nbl32, tree_flags=flags,
                                    bounds=bounds_dev)
     topo._max_cell_depth = max_cell_depth
-    # one read-back for the flags and the level count
-    hv = torch.cat([topo._dev.tree_flags.to(torch.int64).reshape(1),
-                    topo.num_levels.to(torch.int64).reshape(1)]).cpu()
-    if int(hv[0]) & L.FLAG_TIMEOUT:
-        raise L.YgxError("ygx_build_topology: a device-side wait gave up")
-    topo._host = HostTopologyInfo(malformed=bool(int(hv[0]) & L.FLAG_MALFORMED),
-                                  num_levels=int(hv[1]), use_morton=bool(use_morton))
+    if Lf == 1:
+        flag_word, nlev = 0, 1
+    else:
+        nlev, flag_word = tail.tolist()
+        if flag_word & L.FLAG_TIMEOUT:
+            raise L.YgxError("ygx_build_topology: a device-side wait gave up")
+    topo._host = HostTopologyInfo(malformed=bool(flag_word & L.FLAG_MALFORMED),
+                                  num_levels=int(nlev), use_morton=bool(use_morton))
     return topo, pos_sorted, mass_sorted, inv
 
 
