@@ -8,11 +8,21 @@
 // pair (target level, source level, displacement in target-level cells, in
 // float64 exactly as the reference's NumPy code computes it) is packed
 // into a <= 128-bit unsigned key (fields shifted to be non-negative, widths
-// from their ranges), sorted stably with the onesweep sort (low word, then
-// high word carrying the permutation), and the classes are the runs of equal
+// from their ranges), sorted stably, and the classes are the runs of equal
 // keys.
+//
+// The sort is what this costs.  A key of more than 64 bits is sorted by its
+// top 64 alone (8 passes of the onesweep sort); the few pairs that tie there
+// without being of one class (2% of a Plummer tree's pairs, runs of at most a
+// few hundred) are ordered by their remaining bits in place, and only a run
+// too long for that sends the whole list through a sort of the low word first.
+// Beside the sort, the fields are recomputed where they are needed instead of
+// stored (two 62-byte passes over the pairs became one of 24 bytes), each pair
+// travels as one 16-byte record, and the class tables are decoded from the
+// sorted keys.  12,410,462 pairs, 97-bit keys (the far list of 1,048,576
+// Plummer particles): 3.1 -> 2.1 ms.
 #include "common.cuh"
-#include "scan.cuh"
+#include "scan_seg.cuh"
 #include "sort.cuh"
 
 namespace ygx {
@@ -82,32 +92,56 @@ __device__ __forceinline__ double cell_of(double extent, int level) {
   return c > 1e-12 ? c : 1e-12;
 }
 
-// Fields of every pair: target level, source level, displacement index
-// rint((c_t - c_s) / cell(target level)) per axis, in float64; and the
-// per-field minima / maxima (for the key widths).
-__global__ void k_group_fields(const void* src, const void* tgt, int index_bits, int64_t P,
-                               const int32_t* __restrict__ level32,
-                               const float* __restrict__ center, double ex, double ey,
-                               double ez, int32_t* __restrict__ fields,
-                               int* __restrict__ fmin, int* __restrict__ fmax) {
+// The cell sizes of levels 0..63 (a CTA's copy: a division and a scaling less
+// per axis and pair); deeper levels, which tied codes can make, compute theirs.
+struct CellTable {
+  double cell[64][3];
+  __device__ void fill(const double ext[3]) {
+    for (int k = threadIdx.x; k < 64 * 3; k += blockDim.x)
+      cell[k / 3][k % 3] = cell_of(ext[k % 3], k / 3);
+    __syncthreads();
+  }
+  __device__ __forceinline__ double at(int level, int a, const double ext[3]) const {
+    return (unsigned)level < 64u ? cell[level][a] : cell_of(ext[a], level);
+  }
+};
+
+// Fields of a pair: target level, source level, displacement index
+// rint((c_t - c_s) / cell(target level)) per axis, in float64.
+struct GroupPairs {
+  const void *src, *tgt;
+  int index_bits;
+  int64_t P;
+  const int32_t* level32;
+  const float* center;
+  double ext[3];
+};
+__device__ __forceinline__ void group_fields(const GroupPairs& g, const CellTable& cells,
+                                             int64_t s, int64_t t, int v[5]) {
+  v[0] = g.level32[t];
+  v[1] = g.level32[s];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const double delta = (double)g.center[3 * t + a] - (double)g.center[3 * s + a];
+    v[2 + a] = (int)rint(delta / cells.at(v[0], a, g.ext));
+  }
+}
+
+// Minima / maxima of the fields (for the key widths).
+__global__ void k_group_ranges(const GroupPairs g, int* __restrict__ fmin,
+                               int* __restrict__ fmax) {
+  __shared__ CellTable cells;
+  cells.fill(g.ext);
   int lo[5], hi[5];
   for (int f = 0; f < 5; ++f) {
     lo[f] = INT_MAX;
     hi[f] = INT_MIN;
   }
-  const double ext[3] = {ex, ey, ez};
-  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < P;
+  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < g.P;
        p += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t s = load_idx(src, index_bits, p), t = load_idx(tgt, index_bits, p);
     int v[5];
-    v[0] = level32[t];
-    v[1] = level32[s];
-    for (int a = 0; a < 3; ++a) {
-      const double delta = (double)center[3 * t + a] - (double)center[3 * s + a];
-      v[2 + a] = (int)rint(delta / cell_of(ext[a], v[0]));
-    }
+    group_fields(g, cells, load_idx(g.src, g.index_bits, p), load_idx(g.tgt, g.index_bits, p), v);
     for (int f = 0; f < 5; ++f) {
-      fields[5 * p + f] = v[f];
       lo[f] = v[f] < lo[f] ? v[f] : lo[f];
       hi[f] = v[f] > hi[f] ? v[f] : hi[f];
     }
@@ -126,26 +160,91 @@ __global__ void k_group_fields(const void* src, const void* tgt, int index_bits,
   }
 }
 
+// The key: fields from most (0) to least (4) significant; `top` is its upper
+// 64 bits (all of it, if it has no more), `low` the `cut` bits below.
 struct KeyLayout {
   int shift[5];  // bit position of each field in the 128-bit key
   int width[5];
   int fmin[5];
+  int cut;
+};
+struct __align__(16) GroupRec {
+  uint64_t low;
+  int32_t s, t;
 };
 
-__global__ void k_group_pack(const int32_t* __restrict__ fields, int64_t P, KeyLayout kl,
-                             uint64_t* __restrict__ key_lo, uint64_t* __restrict__ key_hi) {
-  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < P;
+__global__ void k_group_pack(const GroupPairs g, KeyLayout kl, KeyLayout* __restrict__ kl_out,
+                             uint64_t* __restrict__ top, GroupRec* __restrict__ rec) {
+  __shared__ CellTable cells;
+  cells.fill(g.ext);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *kl_out = kl;
+  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < g.P;
        p += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t s = load_idx(g.src, g.index_bits, p), t = load_idx(g.tgt, g.index_bits, p);
+    int v[5];
+    group_fields(g, cells, s, t, v);
     unsigned __int128 k = 0;
-    for (int f = 0; f < 5; ++f) {
-      const uint64_t v = (uint64_t)((int64_t)fields[5 * p + f] - (int64_t)kl.fmin[f]);
-      k |= (unsigned __int128)v << kl.shift[f];
-    }
-    key_lo[p] = (uint64_t)k;
-    if (key_hi) key_hi[p] = (uint64_t)(k >> 64);
+    for (int f = 0; f < 5; ++f)
+      k |= (unsigned __int128)(uint64_t)((int64_t)v[f] - (int64_t)kl.fmin[f]) << kl.shift[f];
+    top[p] = (uint64_t)(k >> kl.cut);
+    GroupRec r;
+    r.low = kl.cut > 0 ? (uint64_t)k & (~0ull >> (64 - kl.cut)) : 0ull;
+    r.s = (int32_t)s;
+    r.t = (int32_t)t;
+    rec[p] = r;
   }
 }
 
+// Pairs sorted by `top`: runs of equal words ordered by `low` (stably), out of
+// place.  A warp ranks the runs that start at its 32 positions one after the
+// other, each against itself; runs of more than kTieMax pairs are flagged.
+constexpr int kTieMax = 1024;
+__global__ void k_group_ties(const uint64_t* __restrict__ top, const uint32_t* __restrict__ perm,
+                             const GroupRec* __restrict__ rec, int64_t P,
+                             uint32_t* __restrict__ out, int* __restrict__ too_long) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < P;
+       i0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = i0 + lane;
+    int len = 0;
+    if (i < P && (i == 0 || top[i - 1] != top[i])) {
+      const uint64_t w = top[i];
+      len = 1;
+      while (len <= kTieMax && i + len < P && top[i + len] == w) ++len;
+      if (len == 1) out[i] = perm[i];
+      if (len > kTieMax) *too_long = 1;
+    }
+    unsigned runs = __ballot_sync(0xffffffffu, len > 1 && len <= kTieMax);
+    while (runs) {
+      const int from = __ffs(runs) - 1;
+      runs &= runs - 1;
+      const int64_t a = i0 + from;
+      const int n = __shfl_sync(0xffffffffu, len, from);
+      for (int e0 = 0; e0 < n; e0 += 32) {
+        const int e = e0 + lane;
+        const uint32_t mine = e < n ? perm[a + e] : 0u;
+        const uint64_t low = e < n ? rec[mine].low : 0ull;
+        int rank = 0;
+        for (int j0 = 0; j0 < n; j0 += 32) {
+          const uint64_t theirs = j0 + lane < n ? rec[perm[a + j0 + lane]].low : 0ull;
+          const int m = n - j0 < 32 ? n - j0 : 32;
+          for (int j = 0; j < m; ++j) {
+            const uint64_t v = __shfl_sync(0xffffffffu, theirs, j);
+            rank += v < low || (v == low && j0 + j < e);
+          }
+        }
+        if (e < n) out[a + rank] = mine;
+      }
+    }
+  }
+}
+
+__global__ void k_group_low_keys(const GroupRec* __restrict__ rec, int64_t P,
+                                 uint64_t* __restrict__ out) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < P;
+       i += (int64_t)gridDim.x * blockDim.x)
+    out[i] = rec[i].low;
+}
 __global__ void k_gather_u64(const uint64_t* __restrict__ in, const uint32_t* __restrict__ perm,
                              int64_t n, uint64_t* __restrict__ out) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -153,62 +252,115 @@ __global__ void k_gather_u64(const uint64_t* __restrict__ in, const uint32_t* __
     out[i] = in[perm[i]];
 }
 
-// Run starts of the sorted keys.
-__global__ void k_group_heads(const uint64_t* __restrict__ lo, const uint64_t* __restrict__ hi,
-                              const uint32_t* __restrict__ perm_lo_to_sorted, int64_t P,
-                              int32_t* __restrict__ head) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < P;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    bool h = i == 0;
-    if (!h) {
-      const uint32_t a = perm_lo_to_sorted[i], b = perm_lo_to_sorted[i - 1];
-      h = lo[a] != lo[b] || (hi && hi[a] != hi[b]);
+// Records in sorted order and the run starts (classes), with the number of
+// runs that start in each tile.
+__global__ void __launch_bounds__(kScanThreads)
+    k_group_heads(const uint64_t* __restrict__ top, const uint32_t* __restrict__ perm,
+                  const GroupRec* __restrict__ rec, int64_t P, GroupRec* __restrict__ sorted,
+                  uint8_t* __restrict__ head, int64_t* __restrict__ tile_heads,
+                  const int* __restrict__ skip) {
+  // a run too long to order in place has no permutation here (its entries of
+  // `perm` were not written)
+  if (skip && *skip) return;
+  __shared__ int64_t s_warp[kScanThreads / 32];
+  const int lane = threadIdx.x & 31;
+  const int64_t base = (int64_t)blockIdx.x * kScanTile;
+  int64_t heads = 0;
+  for (int k = 0; k < kScanItems; ++k) {
+    const int64_t i = base + (int64_t)k * kScanThreads + threadIdx.x;
+    GroupRec r{0ull, 0, 0};
+    uint64_t t = 0;
+    if (i < P) {
+      r = rec[perm[i]];
+      t = top[i];
+      sorted[i] = r;
     }
-    head[i] = h ? 1 : 0;
+    uint64_t pl = __shfl_up_sync(0xffffffffu, r.low, 1);
+    if (lane == 0 && i > 0 && i < P) pl = rec[perm[i - 1]].low;
+    if (i < P) {
+      const bool h = i == 0 || top[i - 1] != t || pl != r.low;
+      head[i] = h;
+      heads += h;
+    }
   }
+  heads = seg_block_sum(heads, s_warp);
+  if (threadIdx.x == 0) tile_heads[blockIdx.x] = heads;
 }
 
-__global__ void k_group_emit(const uint32_t* __restrict__ perm, const int32_t* __restrict__ head,
-                             const int64_t* __restrict__ head_scan, int64_t P,
-                             const int32_t* __restrict__ fields, const void* src, const void* tgt,
-                             int index_bits, double ex, double ey, double ez,
-                             int32_t* __restrict__ class_keys, float* __restrict__ class_disp,
-                             void* class_offsets, void* class_sources, void* class_targets,
-                             void* class_ids) {
+__global__ void __launch_bounds__(kScanThreads)
+    k_group_emit(const uint64_t* __restrict__ top, const uint32_t* __restrict__ perm,
+                 const GroupRec* __restrict__ sorted, const uint8_t* __restrict__ head,
+                 const int64_t* __restrict__ tile_off, int64_t P, int index_bits, double ex,
+                 double ey, double ez, const KeyLayout* __restrict__ layout,
+                 int32_t* __restrict__ class_keys, float* __restrict__ class_disp,
+                 void* class_offsets, void* class_sources, void* class_targets,
+                 void* class_ids) {
+  __shared__ KeyLayout kl;
+  __shared__ int s_warp[kScanThreads / 32];
+  if (threadIdx.x == 0) kl = *layout;
+  __syncthreads();
   const double ext[3] = {ex, ey, ez};
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < P;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = perm[i];
-    const int64_t cls = head_scan[i] + head[i] - 1;
-    store_idx(class_sources, index_bits, i, load_idx(src, index_bits, p));
-    store_idx(class_targets, index_bits, i, load_idx(tgt, index_bits, p));
-    // class ids as np.searchsorted(class_starts, arange(n)) (side "left",
-    // grouped_interactions.py:163) gives them: a pair that is not the first
-    // of its class gets the next class's id (a quirk kept for parity)
-    store_idx(class_ids, index_bits, p, head[i] ? cls : cls + 1);
-    if (head[i]) {
-      store_idx(class_offsets, index_bits, cls, i);
-      const int32_t* f = fields + 5 * p;
-      for (int k = 0; k < 5; ++k) class_keys[5 * cls + k] = f[k];
-      for (int a = 0; a < 3; ++a)
-        class_disp[3 * cls + a] = __double2float_rn((double)f[2 + a] * cell_of(ext[a], f[0]));
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t base = (int64_t)blockIdx.x * kScanTile;
+  int64_t before = tile_off[blockIdx.x];
+  for (int k = 0; k < kScanItems; ++k) {
+    const int64_t i = base + (int64_t)k * kScanThreads + threadIdx.x;
+    const bool h = i < P && head[i];
+    const unsigned mask = __ballot_sync(0xffffffffu, h);
+    if (lane == 0) s_warp[warp] = __popc(mask);
+    __syncthreads();
+    int mine = 0, all = 0;
+    for (int w = 0; w < kScanThreads / 32; ++w) {
+      if (w < warp) mine += s_warp[w];
+      all += s_warp[w];
     }
-    if (i == P - 1) store_idx(class_offsets, index_bits, head_scan[P] , P);
+    __syncthreads();
+    if (i < P) {
+      // the class that this pair belongs to: heads up to and including it
+      const int64_t cls =
+          before + mine + __popc(mask & ((2u << lane) - 1u)) - 1;
+      const GroupRec r = sorted[i];
+      store_idx(class_sources, index_bits, i, r.s);
+      store_idx(class_targets, index_bits, i, r.t);
+      // class ids as np.searchsorted(class_starts, arange(n)) (side "left",
+      // grouped_interactions.py:163) gives them: a pair that is not the first
+      // of its class gets the next class's id (a quirk kept for parity)
+      store_idx(class_ids, index_bits, perm[i], h ? cls : cls + 1);
+      if (h) {
+        store_idx(class_offsets, index_bits, cls, i);
+        const unsigned __int128 key = ((unsigned __int128)top[i] << kl.cut) | r.low;
+        int v[5];
+#pragma unroll
+        for (int f = 0; f < 5; ++f) {
+          const uint64_t w = (uint64_t)(key >> kl.shift[f]);
+          v[f] = (int)((int64_t)(kl.width[f] > 0 ? w & (~0ull >> (64 - kl.width[f])) : 0ull) +
+                       (int64_t)kl.fmin[f]);
+          class_keys[5 * cls + f] = v[f];
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+          class_disp[3 * cls + a] = __double2float_rn((double)v[2 + a] * cell_of(ext[a], v[0]));
+      }
+      if (i == P - 1) store_idx(class_offsets, index_bits, cls + 1, P);
+    }
+    before += all;
+    if (base + (int64_t)(k + 1) * kScanThreads >= P) break;
   }
 }
 
 struct GroupScratch {
   int* fmin;
   int* fmax;
-  int32_t* fields;
-  uint64_t* lo;
-  uint64_t* hi;
-  uint64_t* tmp_keys;
-  uint32_t* perm_a;
+  int* too_long;
+  KeyLayout* layout;
+  uint64_t* top;         // pair order
+  uint64_t* top_sorted;
+  GroupRec* rec;         // pair order
+  GroupRec* rec_sorted;
+  uint32_t* perm_a;      // sorted position -> pair
   uint32_t* perm_b;
-  int32_t* head;
-  int64_t* head_scan;
-  int64_t* scan_tmp;
+  uint8_t* head;
+  int64_t* tile_heads;
   SortScratch sort;
 };
 
@@ -217,20 +369,22 @@ GroupScratch carve_group(Arena& a, int64_t P) {
   const int64_t n = P > 0 ? P : 1;
   g.fmin = a.take<int>(8);
   g.fmax = a.take<int>(8);
-  g.fields = a.take<int32_t>(5 * n);
-  g.lo = a.take<uint64_t>(n);
-  g.hi = a.take<uint64_t>(n);
-  g.tmp_keys = a.take<uint64_t>(n);
+  g.too_long = a.take<int>(8);
+  g.layout = a.take<KeyLayout>(1);
+  g.top = a.take<uint64_t>(n);
+  g.top_sorted = a.take<uint64_t>(n);
+  g.rec = a.take<GroupRec>(n);
+  g.rec_sorted = a.take<GroupRec>(n);
   g.perm_a = a.take<uint32_t>(n);
   g.perm_b = a.take<uint32_t>(n);
-  g.head = a.take<int32_t>(n);
-  g.head_scan = a.take<int64_t>(n + 1);
-  g.scan_tmp = a.take<int64_t>(scan_scratch_elems(n));
+  g.head = a.take<uint8_t>(n);
+  g.tile_heads = a.take<int64_t>(scan_tiles(n) + 1);
   g.sort = carve_sort_scratch(a, n);
   return g;
 }
 
-__global__ void k_init_minmax(int* fmin, int* fmax) {
+__global__ void k_init_minmax(int* fmin, int* fmax, int* too_long) {
+  if (threadIdx.x == 0) *too_long = 0;
   if (threadIdx.x < 5) {
     fmin[threadIdx.x] = INT_MAX;
     fmax[threadIdx.x] = INT_MIN;
@@ -299,16 +453,19 @@ int ygx_grouped_classes(const void* sources, const void* targets, int index_bits
   ygx::Arena a{(char*)ws, 0, ws_bytes};
   ygx::GroupScratch g = ygx::carve_group(a, num_pairs);
   const int64_t P = num_pairs;
-  ygx::k_init_minmax<<<1, 32, 0, stream>>>(g.fmin, g.fmax);
+  const ygx::GroupPairs pairs{sources, targets, index_bits,
+                              P,       level32, center,
+                              {root_extent[0], root_extent[1], root_extent[2]}};
+  ygx::k_init_minmax<<<1, 32, 0, stream>>>(g.fmin, g.fmax, g.too_long);
   YGX_CHECK_LAUNCH();
-  ygx::k_group_fields<<<ygx::grid_for(P, 256), 256, 0, stream>>>(
-      sources, targets, index_bits, P, level32, center, root_extent[0], root_extent[1],
-      root_extent[2], g.fields, g.fmin, g.fmax);
+  ygx::k_group_ranges<<<ygx::grid_for(P, 256), 256, 0, stream>>>(pairs, g.fmin, g.fmax);
   YGX_CHECK_LAUNCH();
-  int hmin[8], hmax[8];
-  if (cudaMemcpyAsync(hmin, g.fmin, sizeof(int) * 5, cudaMemcpyDeviceToHost, stream) !=
-          cudaSuccess ||
-      cudaMemcpyAsync(hmax, g.fmax, sizeof(int) * 5, cudaMemcpyDeviceToHost, stream) !=
+  struct {
+    int lo[64], hi[64];  // fmin and fmax lie one arena step apart
+  } range;
+  static_assert(sizeof(range) == 512, "two arena steps");
+  if ((char*)g.fmax - (char*)g.fmin != 256 ||
+      cudaMemcpyAsync(&range, g.fmin, 256 + 5 * sizeof(int), cudaMemcpyDeviceToHost, stream) !=
           cudaSuccess ||
       cudaStreamSynchronize(stream) != cudaSuccess)
     return YGX_ERR_CUDA;
@@ -316,58 +473,68 @@ int ygx_grouped_classes(const void* sources, const void* targets, int index_bits
   ygx::KeyLayout kl;
   int bits = 0;
   for (int f = 4; f >= 0; --f) {
-    kl.fmin[f] = hmin[f];
-    kl.width[f] = ygx::bit_length((uint64_t)((int64_t)hmax[f] - (int64_t)hmin[f]));
+    kl.fmin[f] = range.lo[f];
+    kl.width[f] = ygx::bit_length((uint64_t)((int64_t)range.hi[f] - (int64_t)range.lo[f]));
     kl.shift[f] = bits;
     bits += kl.width[f];
   }
   if (bits > 128) return YGX_ERR_TOO_LARGE;
-  const bool two = bits > 64;
-  ygx::k_group_pack<<<ygx::grid_for(P, 256), 256, 0, stream>>>(g.fields, P, kl, g.lo,
-                                                               two ? g.hi : nullptr);
+  kl.cut = bits > 64 ? bits - 64 : 0;
+  ygx::k_group_pack<<<ygx::grid_for(P, 256), 256, 0, stream>>>(pairs, kl, g.layout, g.top, g.rec);
   YGX_CHECK_LAUNCH();
   uint32_t* status = reinterpret_cast<uint32_t*>(g.fmin + 6);
-  int rc;
-  const uint32_t* perm;  // sorted position -> pair
-  if (bits == 0) {
-    // one class: the identity order
-    rc = ygx::onesweep_sort(g.lo, nullptr, P, 0, 1, g.tmp_keys, g.perm_a, g.sort, false, status,
-                            stream);
-    perm = g.perm_a;
-  } else {
-    rc = ygx::onesweep_sort(g.lo, nullptr, P, 0, two ? 64 : bits, g.tmp_keys, g.perm_a, g.sort,
-                            false, status, stream);
-    perm = g.perm_a;
-    if (!rc && two) {
-      ygx::k_gather_u64<<<ygx::grid_for(P, 256), 256, 0, stream>>>(g.hi, g.perm_a, P, g.lo);
-      YGX_CHECK_LAUNCH();
-      // g.lo now holds the high words in low-word order; sort them carrying perm_a
-      rc = ygx::onesweep_sort(g.lo, g.perm_a, P, 0, bits - 64, g.tmp_keys, g.perm_b, g.sort,
-                              false, status, stream);
-      perm = g.perm_b;
-      // re-pack the low / high words in pair order for the run test
-      if (!rc) {
-        ygx::k_group_pack<<<ygx::grid_for(P, 256), 256, 0, stream>>>(g.fields, P, kl, g.lo, g.hi);
+  const int64_t tiles = ygx::scan_tiles(P);
+  struct {
+    int64_t classes;
+    int too_long;
+  } h{0, 0};
+  // sorted by `top` (one class: the identity order), ties resolved into perm_b;
+  // then, if a run was too long for that, again from a sort by `low`
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    int rc;
+    if (attempt == 0) {
+      rc = ygx::onesweep_sort(g.top, nullptr, P, 0, bits == 0 ? 1 : (bits > 64 ? 64 : bits),
+                              g.top_sorted, kl.cut ? g.perm_a : g.perm_b, g.sort, false, status,
+                              stream);
+      if (rc) return rc;
+      if (kl.cut) {
+        ygx::k_group_ties<<<ygx::grid_for(P, 256), 256, 0, stream>>>(g.top_sorted, g.perm_a, g.rec,
+                                                                     P, g.perm_b, g.too_long);
         YGX_CHECK_LAUNCH();
       }
+    } else {
+      uint64_t* keys = reinterpret_cast<uint64_t*>(g.rec_sorted);  // free until the heads
+      ygx::k_group_low_keys<<<ygx::grid_for(P, 256), 256, 0, stream>>>(g.rec, P, keys);
+      YGX_CHECK_LAUNCH();
+      rc = ygx::onesweep_sort(keys, nullptr, P, 0, kl.cut, g.top_sorted, g.perm_a, g.sort, false,
+                              status, stream);
+      if (rc) return rc;
+      ygx::k_gather_u64<<<ygx::grid_for(P, 256), 256, 0, stream>>>(g.top, g.perm_a, P, keys);
+      YGX_CHECK_LAUNCH();
+      rc = ygx::onesweep_sort(keys, g.perm_a, P, 0, 64, g.top_sorted, g.perm_b, g.sort, false,
+                              status, stream);
+      if (rc) return rc;
     }
+    ygx::k_group_heads<<<(unsigned)tiles, ygx::kScanThreads, 0, stream>>>(
+        g.top_sorted, g.perm_b, g.rec, P, g.rec_sorted, g.head, g.tile_heads,
+        attempt == 0 ? g.too_long : nullptr);
+    YGX_CHECK_LAUNCH();
+    // exclusive over the tiles and, as one more "tile", the total
+    if (cudaMemsetAsync(g.tile_heads + tiles, 0, sizeof(int64_t), stream) != cudaSuccess)
+      return YGX_ERR_CUDA;
+    ygx::k_seg_mid<<<1, 1024, 0, stream>>>(g.tile_heads, tiles + 1);
+    YGX_CHECK_LAUNCH();
+    if (cudaMemcpyAsync(&h.classes, g.tile_heads + tiles, sizeof(int64_t), cudaMemcpyDeviceToHost,
+                        stream) != cudaSuccess ||
+        (kl.cut && attempt == 0 &&
+         cudaMemcpyAsync(&h.too_long, g.too_long, sizeof(int), cudaMemcpyDeviceToHost, stream) !=
+             cudaSuccess) ||
+        cudaStreamSynchronize(stream) != cudaSuccess)
+      return YGX_ERR_CUDA;
+    if (!h.too_long) break;
+    h.too_long = 0;
   }
-  if (rc) return rc;
-  ygx::k_group_heads<<<ygx::grid_for(P, 256), 256, 0, stream>>>(g.lo, two ? g.hi : nullptr, perm,
-                                                                P, g.head);
-  YGX_CHECK_LAUNCH();
-  rc = ygx::exclusive_scan<int32_t>(g.head, P, g.head_scan, g.scan_tmp, stream);
-  if (rc) return rc;
-  int64_t nc = 0;
-  if (cudaMemcpyAsync(&nc, g.head_scan + P, sizeof(int64_t), cudaMemcpyDeviceToHost, stream) !=
-          cudaSuccess ||
-      cudaStreamSynchronize(stream) != cudaSuccess)
-    return YGX_ERR_CUDA;
-  *num_classes_out = nc;
-  if (perm != g.perm_a &&
-      cudaMemcpyAsync(g.perm_a, perm, sizeof(uint32_t) * P, cudaMemcpyDeviceToDevice, stream) !=
-          cudaSuccess)
-    return YGX_ERR_CUDA;
+  *num_classes_out = h.classes;
   return YGX_OK;
 }
 
@@ -382,10 +549,10 @@ int ygx_grouped_emit(const void* sources, const void* targets, int index_bits, i
   if (ws_bytes < ygx_grouped_workspace_size(num_pairs)) return YGX_ERR_ARG;
   ygx::Arena a{(char*)ws, 0, ws_bytes};
   ygx::GroupScratch g = ygx::carve_group(a, num_pairs);
-  ygx::k_group_emit<<<ygx::grid_for(num_pairs, 256), 256, 0, stream>>>(
-      g.perm_a, g.head, g.head_scan, num_pairs, g.fields, sources, targets, index_bits,
-      root_extent[0], root_extent[1], root_extent[2], class_keys, class_disp, class_offsets,
-      class_sources, class_targets, class_ids);
+  ygx::k_group_emit<<<(unsigned)ygx::scan_tiles(num_pairs), ygx::kScanThreads, 0, stream>>>(
+      g.top_sorted, g.perm_b, g.rec_sorted, g.head, g.tile_heads, num_pairs, index_bits,
+      root_extent[0], root_extent[1], root_extent[2], g.layout, class_keys, class_disp,
+      class_offsets, class_sources, class_targets, class_ids);
   YGX_CHECK_LAUNCH();
   return YGX_OK;
 }
