@@ -1192,8 +1192,22 @@ __global__ void k_tw_prefix_copy(const TwPrefix far, const TwPrefix near_,
   for (int64_t x0 = w0 * 1024; x0 < ext_total; x0 += nw * 1024) {
     const int64_t x1 = x0 + 1024 < ext_total ? x0 + 1024 : ext_total;
     int64_t x = x0;
+    int32_t r = tw_row_of(ext_off, rows, x);
     while (x < x1) {
-      const int32_t r = tw_row_of(ext_off, rows, x);
+      // the row that holds x: among the next 64 where many rows overflow, by
+      // search where few do.  4,194,304 clumped particles, fixed depth (58% of
+      // the rows): 257 -> 105 us against a search (20 dependent loads) per row;
+      // passing any distance 32 rows at a time took 444 us instead of 171 on
+      // the 16,777,216-particle Plummer tree (1.3%).
+      unsigned m = 0;
+      for (int tries = 0; tries < 2 && r < rows; ++tries) {
+        const int32_t c = r + lane;
+        m = __ballot_sync(0xffffffffu, c < rows && ext_off[c + 1] > x);
+        if (m) break;
+        r += 32;
+      }
+      r = m ? r + __ffs(m) - 1 : tw_row_of(ext_off, rows, x);
+      if (r >= rows) break;
       const int64_t rb = ext_off[r], re = ext_off[r + 1];
       const int64_t seg_end = re < x1 ? re : x1;
       const unsigned fo = first_ovf[r];
