@@ -693,6 +693,21 @@ int ygx_octree_box_geometry(const uint8_t* valid, const uint64_t* codes, const v
                             const float* bounds_max, float* centers, float* half_extents,
                             float* radii, float* max_extents, cudaStream_t stream);
 
+/* The traversal view of an octree (build_explicit_octree_traversal_view,
+ * octree.py:577-704) in one call on the device: per cell (M) node_of / leaf_of
+ * (index dtype) = the smallest radix node / radix leaf node mapped to it by
+ * node_to_oct (nodes entries) / leaf_to_oct (leaves entries; leaf j is node
+ * num_internal + j), -1 where none or the cell is not valid / not a leaf; the
+ * cell boxes as ygx_octree_box_geometry gives them, from device bounds (3
+ * floats each); counts (device, 2) = valid cells, leaf cells. */
+size_t ygx_octree_view_workspace_size(int64_t M);
+int ygx_octree_view(const uint8_t* valid, const uint8_t* leaf, const uint64_t* codes,
+                    const void* depths, const void* node_to_oct, int64_t nodes,
+                    const void* leaf_to_oct, int64_t leaves, int64_t num_internal, int index_bits,
+                    int64_t M, const float* bounds_min, const float* bounds_max, void* node_of,
+                    void* leaf_of, uint64_t* counts, float* centers, float* half_extents,
+                    float* radii, float* max_extents, void* ws, size_t ws_bytes,
+                    cudaStream_t stream);
 /* _dual_tree_walk_octree_impl (yggdrax/_interactions_impl.py:1908-2597), the
  * walk behind build_octree_native_far_pairs / build_octree_native_neighbor_lists
  * (:5556-5717), in octree cell space from (root, root).  children (M x 8

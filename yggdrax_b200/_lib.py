@@ -65,6 +65,8 @@ _SIGS = {
     "ygx_encode_sort_workspace_size": (SZ, [I64]),
     "ygx_encode_sort": (I32, [P, I64, P, P, P, P, P, SZ, P]),
     "ygx_octree_box_geometry": (I32, [P, P, P, I32, I64, P, P, P, P, P, P, P]),
+    "ygx_octree_view_workspace_size": (SZ, [I64]),
+    "ygx_octree_view": (I32, [P, P, P, P, P, I64, P, I64, I64, I32, I64] + [P] * 10 + [SZ, P]),
     "ygx_octree_walk_workspace_size": (SZ, [I64, I64]),
     "ygx_octree_walk": (I32, [P, P, I32, I64, P, P, P, P, P, P, I64, I64, I32, F32, F32, I64,
                               I64, I64, I64, I64, P, P, P, P, P, P, P, P, P, SZ, P]),

@@ -308,46 +308,106 @@ __device__ __forceinline__ uint64_t compact3(uint64_t x) {
   return x;
 }
 
-// compute_explicit_octree_box_geometry (octree.py:422-476), fp32 with every
-// operation rounded: cell = domain / 2^depth, mins = bmin + cell * index,
-// maxs = mins + cell, centre 0.5 (mins + maxs), half 0.5 (maxs - mins),
-// radius sqrt((h0^2 + h1^2) + h2^2), max extent max(h); zeros on invalid
-// cells.
+// Box of a cell from its code and depth (compute_explicit_octree_box_geometry,
+// octree.py:422-476), fp32 with every operation rounded: cell = domain /
+// 2^depth, mins = bmin + cell * index, maxs = mins + cell, centre 0.5 (mins +
+// maxs), half 0.5 (maxs - mins), radius sqrt((h0^2 + h1^2) + h2^2), max extent
+// max(h); zeros on invalid cells.
+struct OctBoxOut {
+  float *centers, *half, *radii, *max_extents;
+};
+__device__ __forceinline__ void oct_box(int64_t k, bool valid, uint64_t code, int64_t d,
+                                        const float b0[3], const float dom[3],
+                                        const OctBoxOut& o) {
+  float c[3] = {0.f, 0.f, 0.f}, h[3] = {0.f, 0.f, 0.f}, r = 0.f, mx = 0.f;
+  if (valid) {
+    d = d < 0 ? 0 : (d > 21 ? 21 : d);
+    const uint64_t sh = (uint64_t)(21 - d);
+    const uint64_t q[3] = {compact3(code) >> sh, compact3(code >> 1) >> sh,
+                           compact3(code >> 2) >> sh};
+    const float cnt = (float)(1ull << d);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float cell = __fdiv_rn(dom[a], cnt);
+      const float lo = __fadd_rn(b0[a], __fmul_rn(cell, (float)q[a]));
+      const float hi = __fadd_rn(lo, cell);
+      c[a] = __fmul_rn(0.5f, __fadd_rn(lo, hi));
+      h[a] = __fmul_rn(0.5f, __fsub_rn(hi, lo));
+    }
+    const float s = __fadd_rn(__fadd_rn(__fmul_rn(h[0], h[0]), __fmul_rn(h[1], h[1])),
+                              __fmul_rn(h[2], h[2]));
+    r = __fsqrt_rn(s);
+    mx = fmaxf(fmaxf(h[0], h[1]), h[2]);
+  }
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    o.centers[3 * k + a] = c[a];
+    o.half[3 * k + a] = h[a];
+  }
+  o.radii[k] = r;
+  o.max_extents[k] = mx;
+}
+
 __global__ void k_oct_box(const uint8_t* __restrict__ valid, const uint64_t* __restrict__ codes,
                           const void* __restrict__ depths, int index_bits, int64_t M,
                           float bx0, float by0, float bz0, float dx, float dy, float dz,
-                          float* __restrict__ centers, float* __restrict__ half,
-                          float* __restrict__ radii, float* __restrict__ max_extents) {
+                          const OctBoxOut o) {
+  const float b0[3] = {bx0, by0, bz0}, dom[3] = {dx, dy, dz};
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < M;
+       k += (int64_t)gridDim.x * blockDim.x)
+    oct_box(k, valid[k] != 0, codes[k], load_idx(depths, index_bits, k), b0, dom, o);
+}
+
+// The traversal view of an octree (octree.py:577-704): per cell the smallest
+// radix node and radix leaf mapped to it (-1: none, or the cell is not valid /
+// not a leaf), the box, and the numbers of valid and leaf cells.  As tensor
+// operations (two scatters with their index ranges, masks and sums, the bounds
+// read back to the host for the boxes) a view took a quarter of a millisecond;
+// with two launches the octree-native step of 1,048,576 particles (two views)
+// takes 2.61 ms instead of 3.09.
+__global__ void k_oct_view_min(const void* __restrict__ node_to_oct, int64_t nodes,
+                               const void* __restrict__ leaf_to_oct, int64_t leaves,
+                               int64_t first_leaf, int index_bits, int64_t M,
+                               uint32_t* __restrict__ min_node, uint32_t* __restrict__ min_leaf) {
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nodes + leaves;
+       k += (int64_t)gridDim.x * blockDim.x) {
+    const bool node = k < nodes;
+    const int64_t c = node ? load_idx(node_to_oct, index_bits, k)
+                           : load_idx(leaf_to_oct, index_bits, k - nodes);
+    if (c < 0 || c >= M) continue;
+    if (node) atomicMin(min_node + c, (uint32_t)k);
+    else atomicMin(min_leaf + c, (uint32_t)(first_leaf + k - nodes));
+  }
+}
+__global__ void k_oct_view(const uint8_t* __restrict__ valid, const uint8_t* __restrict__ leaf,
+                           const uint64_t* __restrict__ codes, const void* __restrict__ depths,
+                           int index_bits, int64_t M, const float* __restrict__ bmin,
+                           const float* __restrict__ bmax, const uint32_t* __restrict__ min_node,
+                           const uint32_t* __restrict__ min_leaf, void* node_of, void* leaf_of,
+                           unsigned long long* __restrict__ counts, const OctBoxOut o) {
+  float b0[3], dom[3];
+  for (int a = 0; a < 3; ++a) {
+    b0[a] = bmin[a];
+    dom[a] = __fsub_rn(bmax[a], bmin[a]);
+  }
+  unsigned long long nv = 0, nl = 0;
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < M;
        k += (int64_t)gridDim.x * blockDim.x) {
-    float c[3] = {0.f, 0.f, 0.f}, h[3] = {0.f, 0.f, 0.f}, r = 0.f, mx = 0.f;
-    if (valid[k]) {
-      int64_t d = load_idx(depths, index_bits, k);
-      d = d < 0 ? 0 : (d > 21 ? 21 : d);
-      const uint64_t sh = (uint64_t)(21 - d);
-      const uint64_t code = codes[k];
-      const uint64_t q[3] = {compact3(code) >> sh, compact3(code >> 1) >> sh,
-                             compact3(code >> 2) >> sh};
-      const float cnt = (float)(1ull << d);
-      const float b0[3] = {bx0, by0, bz0}, dom[3] = {dx, dy, dz};
-      for (int a = 0; a < 3; ++a) {
-        const float cell = __fdiv_rn(dom[a], cnt);
-        const float lo = __fadd_rn(b0[a], __fmul_rn(cell, (float)q[a]));
-        const float hi = __fadd_rn(lo, cell);
-        c[a] = __fmul_rn(0.5f, __fadd_rn(lo, hi));
-        h[a] = __fmul_rn(0.5f, __fsub_rn(hi, lo));
-      }
-      const float s = __fadd_rn(__fadd_rn(__fmul_rn(h[0], h[0]), __fmul_rn(h[1], h[1])),
-                                __fmul_rn(h[2], h[2]));
-      r = __fsqrt_rn(s);
-      mx = fmaxf(fmaxf(h[0], h[1]), h[2]);
-    }
-    for (int a = 0; a < 3; ++a) {
-      centers[3 * k + a] = c[a];
-      half[3 * k + a] = h[a];
-    }
-    radii[k] = r;
-    max_extents[k] = mx;
+    const bool v = valid[k] != 0, l = leaf[k] != 0;
+    const uint32_t n = min_node[k], f = min_leaf[k];
+    store_idx(node_of, index_bits, k, v && n != 0xffffffffu ? (int64_t)n : -1);
+    store_idx(leaf_of, index_bits, k, l && f != 0xffffffffu ? (int64_t)f : -1);
+    oct_box(k, v, codes[k], load_idx(depths, index_bits, k), b0, dom, o);
+    nv += v;
+    nl += l;
+  }
+  for (int s = 16; s > 0; s >>= 1) {
+    nv += __shfl_xor_sync(0xffffffffu, nv, s);
+    nl += __shfl_xor_sync(0xffffffffu, nl, s);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (nv) atomicAdd(counts, nv);
+    if (nl) atomicAdd(counts + 1, nl);
   }
 }
 
@@ -393,7 +453,43 @@ int ygx_octree_box_geometry(const uint8_t* valid, const uint64_t* codes, const v
               d2 = bounds_max[2] - bounds_min[2];
   ygx::k_oct_box<<<ygx::grid_for(M, 256), 256, 0, stream>>>(
       valid, codes, depths, index_bits, M, bounds_min[0], bounds_min[1], bounds_min[2], d0, d1,
-      d2, centers, half_extents, radii, max_extents);
+      d2, ygx::OctBoxOut{centers, half_extents, radii, max_extents});
+  YGX_CHECK_LAUNCH();
+  return YGX_OK;
+}
+
+size_t ygx_octree_view_workspace_size(int64_t M) {
+  return 2 * ygx::align_up(sizeof(uint32_t) * (size_t)(M > 0 ? M : 1)) + 256;
+}
+
+int ygx_octree_view(const uint8_t* valid, const uint8_t* leaf, const uint64_t* codes,
+                    const void* depths, const void* node_to_oct, int64_t nodes,
+                    const void* leaf_to_oct, int64_t leaves, int64_t num_internal, int index_bits,
+                    int64_t M, const float* bounds_min, const float* bounds_max, void* node_of,
+                    void* leaf_of, uint64_t* counts, float* centers, float* half_extents,
+                    float* radii, float* max_extents, void* ws, size_t ws_bytes,
+                    cudaStream_t stream) {
+  if (M < 1 || M > INT32_MAX || nodes < 0 || nodes > INT32_MAX || leaves < 0 ||
+      num_internal < 0 || num_internal + leaves > INT32_MAX ||
+      (index_bits != 32 && index_bits != 64) || !valid || !leaf || !codes || !depths ||
+      (nodes > 0 && !node_to_oct) || (leaves > 0 && !leaf_to_oct) || !bounds_min ||
+      !bounds_max || !node_of || !leaf_of || !counts || !centers || !half_extents || !radii ||
+      !max_extents || !ws || ws_bytes < ygx_octree_view_workspace_size(M))
+    return YGX_ERR_ARG;
+  ygx::Arena a{(char*)ws, 0, ws_bytes};
+  uint32_t* min_node = a.take<uint32_t>(M);
+  uint32_t* min_leaf = a.take<uint32_t>(M);
+  if (cudaMemsetAsync(min_node, 0xff, (size_t)((char*)(min_leaf + M) - (char*)min_node), stream) !=
+          cudaSuccess ||
+      cudaMemsetAsync(counts, 0, 2 * sizeof(uint64_t), stream) != cudaSuccess)
+    return YGX_ERR_CUDA;
+  ygx::k_oct_view_min<<<ygx::grid_for(nodes + leaves, 256), 256, 0, stream>>>(
+      node_to_oct, nodes, leaf_to_oct, leaves, num_internal, index_bits, M, min_node, min_leaf);
+  YGX_CHECK_LAUNCH();
+  ygx::k_oct_view<<<ygx::grid_for(M, 256), 256, 0, stream>>>(
+      valid, leaf, codes, depths, index_bits, M, bounds_min, bounds_max, min_node, min_leaf,
+      node_of, leaf_of, reinterpret_cast<unsigned long long*>(counts),
+      ygx::OctBoxOut{centers, half_extents, radii, max_extents});
   YGX_CHECK_LAUNCH();
   return YGX_OK;
 }

@@ -154,20 +154,29 @@ def build_explicit_octree_traversal_view(topology) -> ExplicitOctreeTraversalVie
     leaf = t.oct_leaf_mask.to(torch.bool)
     dev = valid.device
     M = int(valid.shape[0])
-    r2o = t.radix_node_to_oct.to(torch.int64)
-    nr = int(r2o.shape[0])
-    o2r = torch.full((M,), nr, dtype=torch.int64, device=dev)
-    o2r.scatter_reduce_(0, r2o, torch.arange(nr, dtype=torch.int64, device=dev), "amin")
-    o2r = torch.where(valid & (o2r < nr), o2r, torch.full_like(o2r, -1))
-    l2o = t.radix_leaf_to_oct.to(torch.int64)
-    ni = int(t.left_child.shape[0])
-    lfill = ni + int(l2o.shape[0])
-    o2l = torch.full((M,), lfill, dtype=torch.int64, device=dev)
-    o2l.scatter_reduce_(0, l2o, torch.arange(ni, lfill, dtype=torch.int64, device=dev), "amin")
-    o2l = torch.where(leaf & (o2l < lfill), o2l, torch.full_like(o2l, -1))
-    box = compute_explicit_octree_box_geometry(valid_mask=valid, node_codes=t.oct_node_codes,
-                                               node_depths=t.oct_node_depths,
-                                               bounds_min=t.bounds_min, bounds_max=t.bounds_max)
+    lib = L.lib()
+    r2o = t.radix_node_to_oct.to(idt).contiguous()
+    l2o = t.radix_leaf_to_oct.to(idt).contiguous()
+    codes = t.oct_node_codes.contiguous()
+    codes = codes.view(torch.int64) if codes.dtype == torch.uint64 else codes.to(torch.int64)
+    depths = t.oct_node_depths.to(idt).contiguous()
+    bmin, bmax = (torch.as_tensor(b).detach().to(device=dev, dtype=torch.float32).contiguous()
+                  for b in (t.bounds_min, t.bounds_max))
+    valid8, leaf8 = (m.to(torch.bool).contiguous().view(torch.uint8) for m in (valid, leaf))
+    o2r, o2l = torch.empty(M, dtype=idt, device=dev), torch.empty(M, dtype=idt, device=dev)
+    counts = torch.empty(2, dtype=torch.int64, device=dev)
+    centers = torch.empty((M, 3), dtype=torch.float32, device=dev)
+    half = torch.empty((M, 3), dtype=torch.float32, device=dev)
+    radii = torch.empty(M, dtype=torch.float32, device=dev)
+    maxe = torch.empty(M, dtype=torch.float32, device=dev)
+    ws = L.workspace(lib.ygx_octree_view_workspace_size(M), dev, zero=False)
+    L.check(lib.ygx_octree_view(
+        L.ptr(valid8), L.ptr(leaf8), L.ptr(codes), L.ptr(depths), L.ptr(r2o), int(r2o.shape[0]),
+        L.ptr(l2o), int(l2o.shape[0]), int(t.left_child.shape[0]), INDEX_BITS, M, L.ptr(bmin),
+        L.ptr(bmax), L.ptr(o2r), L.ptr(o2l), L.ptr(counts), L.ptr(centers), L.ptr(half),
+        L.ptr(radii), L.ptr(maxe), L.ptr(ws), ws.numel(), L.stream_handle(dev)),
+        "ygx_octree_view")
+    counts = counts.to(idt)
     return ExplicitOctreeTraversalView(
         valid_mask=valid, parent=t.oct_parent.to(idt), children=t.oct_children.to(idt),
         child_counts=t.oct_child_counts.to(idt), node_codes=t.oct_node_codes,
@@ -175,10 +184,9 @@ def build_explicit_octree_traversal_view(topology) -> ExplicitOctreeTraversalVie
         nodes_by_level=t.oct_nodes_by_level.to(idt), level_offsets=t.oct_level_offsets.to(idt),
         num_levels=torch.as_tensor(t.oct_num_levels).to(idt), leaf_mask=leaf,
         leaf_nodes=t.oct_leaf_nodes.to(idt), radix_node_to_oct=t.radix_node_to_oct.to(idt),
-        radix_leaf_to_oct=t.radix_leaf_to_oct.to(idt), oct_to_radix_node=o2r.to(idt),
-        oct_to_radix_leaf=o2l.to(idt), num_valid_nodes=valid.sum().to(idt),
-        num_leaf_nodes=leaf.sum().to(idt), box_centers=box.centers,
-        box_half_extents=box.half_extents, box_radii=box.radii, box_max_extents=box.max_extents)
+        radix_leaf_to_oct=t.radix_leaf_to_oct.to(idt), oct_to_radix_node=o2r,
+        oct_to_radix_leaf=o2l, num_valid_nodes=counts[0], num_leaf_nodes=counts[1],
+        box_centers=centers, box_half_extents=half, box_radii=radii, box_max_extents=maxe)
 
 
 def _capacities(tree, max_interactions_per_node, max_neighbors_per_leaf, max_pair_queue,
