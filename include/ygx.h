@@ -417,6 +417,35 @@ int ygx_target_walk_lists(int64_t total, int64_t num_internal, const int64_t* ca
                           const int32_t* leafpos32, int64_t max_nbr,
                           void* neighbor_leaf_positions, void* ws, size_t ws_bytes,
                           cudaStream_t stream);
+/* The per-target walk over a batched forest (ygx_batch_build_topology: global
+ * node ids, set q's nodes from 2 leaf_off[q] - q on): unordered, without
+ * predicted rows, forests of at most 2^23 nodes.  caps / needs_out / stats_out
+ * / flags_out as for ygx_target_walk (the queue holds 2 entries per set and one
+ * per internal node that is no root); YGX_FLAG_MALFORMED: a set has tied leaf
+ * codes, use ygx_batch_traverse_walk.  ygx_batch_target_walk_lists then gives
+ * the rows as ygx_traverse_finalize does: far rows in nbl32 order, near rows by
+ * leaf position, far_row_base / near_row_base (int32 per row, may be null)
+ * subtracted from every id.  Both on one workspace; the first synchronizes. */
+size_t ygx_batch_target_walk_workspace_size(int64_t total, int64_t num_leaves,
+                                            const int64_t* caps);
+int ygx_batch_target_walk(const float* center, const float* radius, const float* max_extent,
+                          const int32_t* left32, const int32_t* right32,
+                          const int32_t* leafpos32, const int32_t* level32, int64_t total,
+                          int64_t num_leaves, const int64_t* leaf_off, int64_t S,
+                          const uint32_t* seg_flags, int mac, float theta,
+                          float dehnen_radius_scale, const int64_t* caps, uint64_t* stats_out,
+                          uint64_t* needs_out, uint32_t* flags_out, void* ws, size_t ws_bytes,
+                          cudaStream_t stream);
+int ygx_batch_target_walk_lists(int64_t total, int64_t num_leaves, const int64_t* caps,
+                                int32_t* far_raw, int64_t far_raw_cap, int32_t* near_raw,
+                                int64_t near_raw_cap, const int32_t* nbl32,
+                                const int32_t* level32, const int32_t* far_row_base,
+                                const int32_t* near_row_base, int index_bits, int64_t far_total,
+                                int64_t near_total, uint64_t far_records, uint64_t near_records,
+                                void* node_offsets, void* far_counts, void* sources,
+                                void* targets, void* target_levels, void* near_offsets,
+                                void* near_counts, void* neighbors, void* ws, size_t ws_bytes,
+                                cudaStream_t stream);
 /* Padded row slots for predicted capacities (no reference counterpart: the
  * reference sizes rows by its count pass): pad_far[0..total] /
  * pad_near[0..num_leaves] = exclusive sums of far_rcap32 / near_rcap32 (int64,

@@ -27,8 +27,10 @@ import torch
 from . import _lib as L
 from .dtypes import INDEX_BITS, INDEX_DTYPE
 from .geometry import TreeGeometry
-from .interactions import (_CAPACITY_HINTS, _MAC_CODES, _WF_CAP_MAX, NodeInteractionList,
-                           NodeNeighborList, _dense_neighbor_budget, _grow_wf_cap, _hint_key)
+from .interactions import (_CAPACITY_HINTS, _MAC_CODES, _PAIR_WALK_MAX_NODES, _TARGET_HINTS,
+                           _WF_CAP_MAX, NodeInteractionList, NodeNeighborList,
+                           _dense_neighbor_budget, _grow_target_caps, _grow_wf_cap, _hint_key,
+                           _target_caps)
 from .tree import MAX_TREE_LEVELS, RadixTreeTopology
 
 _GENS_HINTS_BATCH: dict = {}
@@ -365,11 +367,98 @@ def build_interactions_and_neighbors_batched(batch: BatchedTrees, geometry: Batc
                                              dehnen_radius_scale: float = 1.0
                                              ) -> BatchedInteractions:
     """The exact far / near lists (count-then-fill semantics, no capacities)
-    of every set, from one walk over the whole forest."""
+    of every set, from one walk over the whole forest: the per-target walk
+    (512 sets of 256 to 65,536 particles: 4.6 -> 3.1 ms of GPU time against
+    the generation walk and its log's scatter), or for forests it does not serve (tied
+    leaf codes, more than 2^23 nodes) the generation walk."""
     if mac_type not in _MAC_CODES:
         raise ValueError(f"Unknown mac_type '{mac_type}'")
     if float(dehnen_radius_scale) <= 0.0:
         raise ValueError("dehnen_radius_scale must be > 0")
+    total = batch.total_nodes
+    if total >= 3 and batch.total_leaves > batch.num_sets and 2 * total <= _PAIR_WALK_MAX_NODES:
+        out = _target_lists_batched(batch, geometry, theta, mac_type, dehnen_radius_scale)
+        if out is not None:
+            return out
+    return _log_lists_batched(batch, geometry, theta, mac_type, dehnen_radius_scale)
+
+
+# First capacities of a forest's per-target walk, entries per node (far, near
+# and split entries, continuations, records of the three, queue): sets of up
+# to some 20,000 particles fit, and 8 M nodes take 14 GB; what a walk needed
+# then sizes the next one.
+_BATCH_FIRST_CAPS = [84.0, 140.0, 140.0, 14.0, 6.0, 6.0, 6.0, 4.0]
+
+
+def _target_lists_batched(batch: BatchedTrees, geometry: BatchedGeometry, theta: float,
+                          mac_type: str, dehnen_radius_scale: float):
+    """ygx_batch_target_walk + ygx_batch_target_walk_lists; None when a set is
+    malformed or the walk gave up (then the caller runs the generation walk)."""
+    lib = L.lib()
+    dev = batch.parent.device
+    st = L.stream_handle(dev)
+    ib, idt = INDEX_BITS, INDEX_DTYPE
+    total, Lt, S = batch.total_nodes, batch.total_leaves, batch.num_sets
+    center = geometry.center.contiguous()
+    radius = geometry.radius.contiguous()
+    max_extent = geometry.max_extent.contiguous()
+    key = _hint_key(mac_type, theta, total, "batch_target")
+    caps = _target_caps(total, Lt, _TARGET_HINTS.get(key, _BATCH_FIRST_CAPS))
+    runs = 0
+    while True:
+        runs += 1
+        caps_np = np.asarray(caps, np.int64)
+        ws = L.workspace(lib.ygx_batch_target_walk_workspace_size(total, Lt, caps_np.ctypes.data),
+                         dev, zero=False)
+        stats = np.zeros(L.TSTAT_WORDS, np.uint64)
+        needs = np.zeros(14, np.uint64)
+        flags = np.zeros(1, np.uint32)
+        L.check(lib.ygx_batch_target_walk(
+            L.ptr(center), L.ptr(radius), L.ptr(max_extent), L.ptr(batch.left32),
+            L.ptr(batch.right32), L.ptr(batch.leafpos32), L.ptr(batch.level32), total, Lt,
+            L.ptr(batch.leaf_off), S, L.ptr(batch.seg_flags), _MAC_CODES[mac_type], float(theta),
+            float(dehnen_radius_scale), caps_np.ctypes.data, stats.ctypes.data,
+            needs.ctypes.data, flags.ctypes.data, L.ptr(ws), ws.numel(), st),
+            "ygx_batch_target_walk")
+        f = int(flags[0])
+        if f & L.FLAG_BAD_INPUT:
+            raise ValueError("MAC extents must be positive (geometry has zero or NaN extents)")
+        if f & (L.FLAG_TIMEOUT | L.FLAG_MALFORMED):
+            return None
+        if f & L.FLAG_LOG_OVERFLOW:
+            caps = _grow_target_caps(caps, needs, runs, f)
+            ws = None
+            continue
+        if f:
+            raise L.YgxError(f"target walk reported flags {f:#x}")
+        break
+    prev = _TARGET_HINTS.get(key)
+    cur = [int(n) / total for n in needs[:8]]
+    _TARGET_HINTS[key] = cur if prev is None else [max(a, b) for a, b in zip(prev, cur)]
+    s = {k: int(stats[v]) for k, v in L.TSTAT.items()}
+    P, Q = s["far_total"], s["near_total"]
+    e = lambda k, dt=idt: torch.empty(k, dtype=dt, device=dev)  # noqa: E731
+    far_raw, near_raw = e(max(P, 1), torch.int32), e(max(Q, 1), torch.int32)
+    out = BatchedInteractions(
+        node_offsets=e(total + 1), far_counts=e(total), sources=e(P), targets=e(P),
+        target_levels=e(P), near_offsets=e(Lt + 1), near_counts=e(Lt), neighbors=e(Q), stats=s)
+    L.check(lib.ygx_batch_target_walk_lists(
+        total, Lt, caps_np.ctypes.data, L.ptr(far_raw), far_raw.numel(), L.ptr(near_raw),
+        near_raw.numel(), L.ptr(batch.nbl32), L.ptr(batch.level32), L.ptr(batch.node_base32),
+        L.ptr(batch.leaf_base32), ib, P, Q, int(needs[4]), int(needs[5]),
+        L.ptr(out.node_offsets), L.ptr(out.far_counts), L.ptr(out.sources), L.ptr(out.targets),
+        L.ptr(out.target_levels), L.ptr(out.near_offsets), L.ptr(out.near_counts),
+        L.ptr(out.neighbors), L.ptr(ws), ws.numel(), st), "ygx_batch_target_walk_lists")
+    f = L.read_status(ws)
+    if f:
+        raise L.YgxError(f"target walk lists reported flags {f:#x}")
+    return out
+
+
+def _log_lists_batched(batch: BatchedTrees, geometry: BatchedGeometry, theta: float,
+                       mac_type: str, dehnen_radius_scale: float) -> BatchedInteractions:
+    """The generation walk with its pair log (whose sizes BatchedPipeline's
+    graph is captured with)."""
     lib = L.lib()
     dev = batch.parent.device
     st = L.stream_handle(dev)
@@ -525,9 +614,7 @@ class BatchedPipeline:
     def _eager(self, positions, masses):
         bt = _build_on_layout(positions, masses, self.layout)
         bg = compute_tree_geometry_batched(bt)
-        bi = build_interactions_and_neighbors_batched(
-            bt, bg, theta=self.theta, mac_type=self.mac_type,
-            dehnen_radius_scale=self.scale)
+        bi = _log_lists_batched(bt, bg, self.theta, self.mac_type, self.scale)
         st = bi.stats
         if st:
             m = self.margin

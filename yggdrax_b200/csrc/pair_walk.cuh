@@ -29,6 +29,9 @@
 //    1,000,003 Plummer, leaf 32                1.50 -> 0.78 ms   2.0 -> 1.1 M
 //       65,536 cube, leaf 16                   0.37 -> 0.19 ms
 //        4,000 cube, leaf 8, bh 0.5            0.18 -> 0.08 ms
+// A forest of 512 sets of 256 to 65,536 particles (leaf 16, dehnen 0.6)
+// walks in 2.64 ms and its rows are copied in 0.49, where the generation walk took 2.93 and its log's scatter
+// 1.70.
 // The large trees are bound by instruction issue, the small ones by the chain
 // of dependent gathers down the tree's levels.  Pairs evaluated 32 wide with
 // the next window prefetched took 8.3 ms at 16M; 5 CTAs per SM spill (8.0).
@@ -47,6 +50,10 @@ constexpr int kPwInhGroup = 64;    // inherited candidates per continuation piec
 constexpr uint32_t kPwSlotMask = 0xffffffu;
 constexpr uint32_t kPwGen = 0x1000000u;
 constexpr int64_t kPwMaxNodes = 1 << 24;  // slots are 24 bits
+// A forest's nodes are not internal nodes first, so a slot's id says itself
+// whether it is a leaf: its sign bit, which the lists' copies drop.
+constexpr uint32_t kPwLeaf = 0x80000000u;
+constexpr uint32_t kPwId = 0x7fffffffu;
 
 enum PwFlag : uint32_t { kPwSibling = 1u, kPwShared = 2u };
 
@@ -86,9 +93,10 @@ struct PwSmem {
 
 struct PwArgs {
   const float4* sc;        // per slot: centre x, y, z and MAC extent
-  const int32_t* sid;      // per slot: node id
-  const PwRow* rows;       // far rows per node, then near rows per leaf id
-  int32_t ni, n_targets;
+  const int32_t* sid;      // per slot: node id, kPwLeaf set on leaves
+  const PwRow* rows;       // far rows per node
+  const PwRow* near_rows;  // near rows per node (leaves only)
+  int32_t n_targets;
   float theta_sq, theta;
   // per node, zeroed; used only by targets that were handed off
   int32_t* s_cnt;
@@ -196,7 +204,8 @@ __global__ void k_pw_slots(const float* __restrict__ center, const float* __rest
     // dereferenced as a node (a leaf id ends the walk there)
     if (!(r.w > 0.0f)) raise_flag(status, kFlagBadInput);
     sc[s] = r;
-    sid[s] = (unsigned)c < (unsigned)total ? c : total - 1;
+    const int32_t id = (unsigned)c < (unsigned)total ? c : total - 1;
+    sid[s] = id >= ni ? (int32_t)((uint32_t)id | kPwLeaf) : id;
     if (s < 2) {
       if (s == 0) {
         float e = mac == kTwBH ? max_extent[root] : radius[root];
@@ -213,6 +222,81 @@ __global__ void k_pw_slots(const float* __restrict__ center, const float* __rest
       q_ready[s] = 1u;
     }
   }
+}
+
+// The same for a forest (batched sets; set q's nodes from 2 leaf_off[q] - q on,
+// its root first), a thread per node, bound by its gathers of two children
+// (12 us for 512 sets of 256 to 65,536 particles): slots of every internal node by
+// global id, rows without predicted slots, the two pieces of every set with a
+// pair, and the nodes per level of all sets.  A set with tied codes is
+// flagged: the host then runs the generation walk.
+__global__ void k_pw_forest_slots(const float* __restrict__ center,
+                                  const float* __restrict__ radius,
+                                  const float* __restrict__ max_extent,
+                                  const int32_t* __restrict__ left32,
+                                  const int32_t* __restrict__ right32,
+                                  const int32_t* __restrict__ leafpos,
+                                  const int32_t* __restrict__ level32, int32_t total,
+                                  const int64_t* __restrict__ leaf_off, int64_t S,
+                                  const uint32_t* __restrict__ seg_flags, int mac,
+                                  float dehnen_scale, float4* __restrict__ sc,
+                                  int32_t* __restrict__ sid, PwPiece* __restrict__ queue,
+                                  unsigned int* __restrict__ q_ready, unsigned int q_cap,
+                                  TwCtl* __restrict__ ctl, PwRow* __restrict__ rows,
+                                  PwRow* __restrict__ near_rows, int64_t* __restrict__ levels,
+                                  uint32_t* __restrict__ status) {
+  __shared__ unsigned s_levels[kTwHist / 2];
+  for (int k = threadIdx.x; k < kTwHist / 2; k += blockDim.x) s_levels[k] = 0;
+  __syncthreads();
+  auto extent = [&](int32_t v) {  // _build_mac_extents (_interactions_impl.py:993-1061)
+    const float e = mac == kTwBH ? max_extent[v] : radius[v];
+    return mac == kTwDehnen ? __fmul_rn(dehnen_scale, e) : e;
+  };
+  for (int32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < total; k += gridDim.x * blockDim.x) {
+    rows[k] = PwRow{0, 0, k};
+    if (!(extent(k) > 0.0f)) raise_flag(status, kFlagBadInput);
+    const int lv = level32[k];
+    atomicAdd(&s_levels[lv < 0 ? 0 : lv < kTwHist / 2 ? lv : kTwHist / 2 - 1], 1u);
+    const int32_t ch[2] = {left32[k], right32[k]};
+    if (ch[0] < 0) {
+      near_rows[k] = PwRow{0, 0, leafpos[k]};
+      continue;
+    }
+    for (int side = 0; side < 2; ++side) {
+      const int32_t c = ch[side];
+      const bool in = (unsigned)c < (unsigned)total;
+      if (!in) raise_flag(status, kFlagBadInput);  // ends there, as a leaf (see k_pw_slots)
+      sc[2 * k + side] = in ? make_float4(center[3 * c], center[3 * c + 1], center[3 * c + 2],
+                                          extent(c))
+                            : make_float4(0.f, 0.f, 0.f, 0.f);
+      sid[2 * k + side] = !in || left32[c] < 0 ? (int32_t)((uint32_t)(in ? c : k) | kPwLeaf) : c;
+    }
+  }
+  for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < S;
+       q += (int64_t)gridDim.x * blockDim.x) {
+    if (leaf_off[q + 1] - leaf_off[q] < 2) continue;
+    if (seg_flags[q] & kFlagMalformed) {  // no tree to walk: nothing of it is queued
+      raise_flag(status, kFlagMalformed);
+      ctl->stop = 1u;
+      ctl->q_head = q_cap;  // no warp takes a piece of any set
+      continue;
+    }
+    const uint32_t root = (uint32_t)(2 * leaf_off[q] - q);
+    const unsigned at = atomicAdd(&ctl->q_tail, 2u);
+    if (at + 2u > q_cap) {
+      raise_flag(status, kFlagLogOverflow);
+      ctl->stop = 1u;
+      continue;
+    }
+    for (uint32_t side = 0; side < 2; ++side) {
+      queue[at + side] = PwPiece{(2u * root + side) | kPwGen, kPwSibling, 0u, 0u, 0ull, 0ull};
+      q_ready[at + side] = 1u;
+    }
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < kTwHist / 2; k += blockDim.x)
+    if (s_levels[k])
+      atomicAdd(reinterpret_cast<unsigned long long*>(levels) + k, (unsigned long long)s_levels[k]);
 }
 
 // Warp-collective: n staged ids of one row to the row's predicted slot where
@@ -238,7 +322,7 @@ __device__ __noinline__ void pw_flush_row(const PwArgs& a, PwWarpSmem& W, int ne
   within = __shfl_sync(0xffffffffu, within, 0);
   if ((long long)within + n <= (long long)R.rcap) {
     int32_t* raw = (near ? a.near_raw : a.far_raw) + R.pad + within;
-    for (int k = lane; k < n; k += 32) raw[k] = (int32_t)stg[k];
+    for (int k = lane; k < n; k += 32) raw[k] = (int32_t)(stg[k] & kPwId);
     return;
   }
   unsigned long long off = 0, ri = 0;
@@ -255,7 +339,7 @@ __device__ __noinline__ void pw_flush_row(const PwArgs& a, PwWarpSmem& W, int ne
     return;
   }
   int32_t* pool = near ? a.near_pool : a.far_pool;
-  for (int k = lane; k < n; k += 32) pool[off + k] = (int32_t)stg[k];
+  for (int k = lane; k < n; k += 32) pool[off + k] = (int32_t)(stg[k] & kPwId);
   if (lane == 0) {
     (near ? a.near_keys : a.far_keys)[ri] =
         ((unsigned long long)(uint32_t)R.row << 32) | (unsigned long long)(uint32_t)within;
@@ -499,8 +583,8 @@ __device__ __forceinline__ bool pw_accept(const float4 T, const float4 c, const 
 // Internal target: it splits itself unless the source is larger (canonical
 // orientation, :1444-1454: the lower id splits on a tie).
 template <bool kLeaf>
-__device__ __forceinline__ bool pw_keep(int t, float et, int s, float es, int ni) {
-  const bool s_leaf = s >= ni;
+__device__ __forceinline__ bool pw_keep(int t, float et, int s, float es) {
+  const bool s_leaf = s < 0;  // kPwLeaf
   return kLeaf ? s_leaf : (s_leaf || (t < s ? et >= es : !(es >= et)));
 }
 
@@ -556,8 +640,8 @@ __device__ __forceinline__ bool pw_run_piece(const PwArgs& a, PwSmem& sm, PwWarp
     if (act1) atomicAdd(&sm.hist[e1 >> 24], 1u);
     const bool a0 = act0 && pw_accept<kMac>(Tc, c0, a);
     const bool a1 = act1 && pw_accept<kMac>(Tc, c1, a);
-    const bool b0 = act0 && !a0 && pw_keep<kLeaf>(t, Tc.w, s0, c0.w, a.ni);
-    const bool b1 = act1 && !a1 && pw_keep<kLeaf>(t, Tc.w, s1, c1.w, a.ni);
+    const bool b0 = act0 && !a0 && pw_keep<kLeaf>(t, Tc.w, s0, c0.w);
+    const bool b1 = act1 && !a1 && pw_keep<kLeaf>(t, Tc.w, s1, c1.w);
     const bool r0 = act0 && !a0 && !b0, r1 = act1 && !a1 && !b1;
     // (the ballots also order this window's stack reads before the pushes)
     const unsigned mR0 = __ballot_sync(0xffffffffu, r0), mR1 = __ballot_sync(0xffffffffu, r1);
@@ -691,8 +775,9 @@ __global__ void __launch_bounds__(kPwThreads, kPwBlocksPerSM)
     have = false;
     const uint32_t slot = pc.et & kPwSlotMask;
     const float4 Tc = __ldg(a.sc + slot);
-    const int t = __ldg(a.sid + slot);
-    const bool t_leaf = t >= a.ni;
+    const int t_id = __ldg(a.sid + slot);
+    const bool t_leaf = t_id < 0;
+    const int t = t_id & (int)kPwId;
     if (lane == 0) {
       const long long now = clock64();
       W.st.idle += (unsigned long long)(now - W.t_mark);
@@ -703,7 +788,7 @@ __global__ void __launch_bounds__(kPwThreads, kPwBlocksPerSM)
       W.s_len = 0;
       // the rows' places arrive while the first candidates are evaluated
       pw_copy16(&W.row[0], a.rows + t);
-      if (t_leaf) pw_copy16(&W.row[1], a.rows + a.n_targets + 1 + (t - a.ni));
+      if (t_leaf) pw_copy16(&W.row[1], a.near_rows + t);
     }
     __syncwarp();
     const bool shared = t_leaf ? pw_run_piece<kMac, true>(a, sm, W, pc, t, Tc, lane, lt)

@@ -1391,7 +1391,8 @@ struct TwScratch {
 // needs its candidates in Morton order, and larger trees need wider ids.
 static bool use_pairs(int64_t total, bool ordered) { return !ordered && total <= kPwMaxNodes; }
 
-static TwScratch carve_tw(Arena& a, int64_t total, int64_t L, const TwCaps& c, bool ordered) {
+static TwScratch carve_tw(Arena& a, int64_t total, int64_t L, const TwCaps& c, bool ordered,
+                          bool forest = false) {
   TwScratch s{};
   const bool pairs = use_pairs(total, ordered);
   // status word, control block, histogram and row stats first: one memset
@@ -1411,12 +1412,13 @@ static TwScratch carve_tw(Arena& a, int64_t total, int64_t L, const TwCaps& c, b
   // per node, written before use
   s.s_head = a.take<int32_t>(total);
   if (pairs) {
-    s.sc = a.take<float4>(total);
-    s.sid = a.take<int32_t>(total);
+    // (a forest's slots are two per node, its near rows one per node)
+    s.sc = a.take<float4>(forest ? 2 * total : total);
+    s.sid = a.take<int32_t>(forest ? 2 * total : total);
     s.s_pool32 = a.take<uint32_t>(c.split);
     s.spill32 = a.take<uint32_t>(c.spill);
     s.queue32 = a.take<PwPiece>(c.queue);
-    s.pw_rows = a.take<PwRow>(total + L);
+    s.pw_rows = a.take<PwRow>(forest ? 2 * total : total + L);
   } else {
     s.recs = a.take<TwRec>(total);
     s.first = a.take<int32_t>(total);
@@ -1460,6 +1462,156 @@ static TwScratch carve_tw(Arena& a, int64_t total, int64_t L, const TwCaps& c, b
     s.rs = carve_row_sort(a, total, L);
   }
   return s;
+}
+
+// Pool blocks a warp claims: small enough that every warp's open blocks fit
+// the pools many times over, large enough to keep the global cursors quiet.
+struct TwBlocks {
+  unsigned long long entries;
+  unsigned records;
+  explicit TwBlocks(const TwCaps& c) {
+    const long long nwarps = (long long)kNumSMs * kTwBlocksPerSM * kTwWarps;
+    long long me = c.far < c.near_ ? c.far : c.near_;
+    me = me < c.split ? me : c.split;
+    const long long be = me / (nwarps * 16);
+    entries = (unsigned long long)(be < 32 ? 32 : (be > 2048 ? 2048 : be));
+    long long mr = c.far_rec < c.near_rec ? c.far_rec : c.near_rec;
+    mr = mr < c.s_rec ? mr : c.s_rec;
+    const long long br = mr / (nwarps * 8);
+    records = (unsigned)(br < 4 ? 4 : (br > 64 ? 64 : br));
+  }
+};
+
+// The pair walk's arguments but for the rows' places.
+static PwArgs pair_args(const TwScratch& s, const TwCaps& c, int32_t targets, float theta) {
+  PwArgs a{};
+  a.sc = s.sc;
+  a.sid = s.sid;
+  a.n_targets = targets;
+  a.theta_sq = theta * theta;
+  a.theta = sqrtf(a.theta_sq);
+  a.s_cnt = s.s_cnt;
+  a.s_nch = s.s_nch;
+  a.s_head = s.s_head;
+  a.pieces_left = s.pieces_left;
+  a.far_cnt = s.far_cnt;
+  a.near_cnt = s.near_cnt;
+  a.far_pool = s.far_pool;
+  a.near_pool = s.near_pool;
+  a.s_pool = s.s_pool32;
+  a.spill = s.spill32;
+  a.far_cap = (unsigned long long)c.far;
+  a.near_cap = (unsigned long long)c.near_;
+  a.s_cap = (unsigned long long)c.split;
+  a.spill_cap = (unsigned long long)c.spill;
+  a.far_keys = s.far_keys;
+  a.far_recs = s.far_recs;
+  a.near_keys = s.near_keys;
+  a.near_recs = s.near_recs;
+  a.s_recs = s.s_recs;
+  a.far_rec_cap = (unsigned)c.far_rec;
+  a.near_rec_cap = (unsigned)c.near_rec;
+  a.s_rec_cap = (unsigned)c.s_rec;
+  a.q_cap = (unsigned)c.queue;
+  a.queue = s.queue32;
+  a.q_ready = s.q_ready;
+  a.gen_hist = s.gen_hist;
+  a.ctl = s.ctl;
+  a.status = s.status;
+  a.spin_limit = (uint32_t)g_tune.spin_limit;
+  a.budget = g_tune.target_budget;
+  const TwBlocks blk(c);
+  a.blk_entries = blk.entries;
+  a.blk_records = blk.records;
+  return a;
+}
+
+static cudaError_t launch_pair_walk(PwArgs a, int mac, int64_t total, cudaStream_t stream) {
+  const size_t smem = sizeof(PwSmem);
+  static std::atomic<uint64_t> attr[3];
+  // a small tree never has work for every warp of the device; fewer CTAs
+  // start and end sooner
+  const int grid = grid_for(total, 16, kNumSMs * kPwBlocksPerSM);
+  a.hungry = grid * kPwWarps / 4;
+  cudaError_t e;
+#define YGX_PW(M)                                                                    \
+  e = ensure_smem_limit(k_pair_walk<M>, (int)smem, attr[M]);                         \
+  if (e == cudaSuccess) k_pair_walk<M><<<grid, kPwThreads, smem, stream>>>(a)
+  switch (mac) {
+    case kTwBH: YGX_PW(kTwBH); break;
+    case kTwDehnen: YGX_PW(kTwDehnen); break;
+    default: YGX_PW(kTwEngblom); break;
+  }
+#undef YGX_PW
+  return e;
+}
+
+// What the host reads after a walk (status word to levels lie one behind the
+// other: one read), and the statistics it makes of it.  Synchronizes.
+struct TwRead {
+  uint32_t flags;
+  TwCtl ctl;
+  unsigned int hist[kTwHist];
+  unsigned long long rs[8];
+  int64_t levels[kTwHist / 2 + 1];
+};
+static int read_walk(const TwScratch& s, TwRead* r, cudaStream_t stream) {
+  alignas(16) char block[8192];
+  const char* first = (const char*)s.status;
+  const size_t bytes = (const char*)(s.levels + kTwHist / 2 + 1) - first;
+  if (bytes > sizeof(block)) return YGX_ERR_ARG;
+  if (cudaMemcpyAsync(block, first, bytes, cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+      cudaStreamSynchronize(stream) != cudaSuccess)
+    return YGX_ERR_CUDA;
+  auto at = [&](const void* p) { return block + ((const char*)p - first); };
+  memcpy(&r->flags, at(s.status), sizeof(uint32_t));
+  memcpy(&r->ctl, at(s.ctl), sizeof(r->ctl));
+  memcpy(r->hist, at(s.gen_hist), sizeof(r->hist));
+  memcpy(r->rs, at(s.rowstat), sizeof(r->rs));
+  memcpy(r->levels, at(s.levels), sizeof(r->levels));
+  return YGX_OK;
+}
+// level_count[l]: nodes of level l.  Every node's self pair {v, v} sits at
+// generation depth(v); every other pair was evaluated once from each side.
+static void walk_stats(const TwRead& r, const int64_t* level_count, int num_levels, int64_t total,
+                       bool pred, uint64_t* stats_out, uint64_t* needs_out) {
+  unsigned long long wf2[kTwHist];
+  for (int g = 0; g < kTwHist; ++g) wf2[g] = r.hist[g];
+  for (int l = 0; l < num_levels && l < kTwHist; ++l)
+    wf2[l] += 2ull * (unsigned long long)level_count[l];
+  unsigned long long mw = 1, gens = 0;
+  for (int g = 0; g < kTwHist; ++g) {
+    if (wf2[g] == 0) continue;
+    gens = (unsigned long long)g + 1;
+    if (g > 0 && wf2[g] / 2 > mw) mw = wf2[g] / 2;
+  }
+  const TwCtl& ctl = r.ctl;
+  const unsigned long long* rs = r.rs;
+  for (int k = 0; k < YGX_TSTAT_WORDS; ++k) stats_out[k] = 0;
+  stats_out[YGX_TSTAT_FAR_TOTAL] = rs[0];
+  stats_out[YGX_TSTAT_NEAR_TOTAL] = rs[1];
+  stats_out[YGX_TSTAT_MAX_FAR] = rs[2];
+  stats_out[YGX_TSTAT_MAX_NEAR] = rs[3];
+  stats_out[YGX_TSTAT_ACCEPT] = ctl.acc_sides / 2;
+  stats_out[YGX_TSTAT_NEAR] = ctl.near_sides / 2;
+  stats_out[YGX_TSTAT_REFINE] = ctl.ref_sides / 2 + (unsigned long long)total;
+  stats_out[YGX_TSTAT_MAX_WF] = mw;
+  stats_out[YGX_TSTAT_GENS] = gens;
+  if (pred) {
+    stats_out[YGX_TSTAT_OVF_ROWS] = rs[4];
+    stats_out[YGX_TSTAT_OVF_ENTRIES] = rs[5];
+    stats_out[YGX_TSTAT_EXT_FAR] = rs[6];
+    stats_out[YGX_TSTAT_EXT_NEAR] = rs[7];
+  }
+  // what each capacity needed (a re-run with these fits)
+  const uint64_t needs[14] = {ctl.far_cur,     ctl.near_cur,    ctl.s_cur,
+                              ctl.spill_cur,   ctl.far_rec_cur, ctl.near_rec_cur,
+                              ctl.s_rec_cur,   ctl.q_tail,      ctl.max_cmp,
+                              // warp cycles on pieces / waiting, pieces run,
+                              // steps and the candidates they held
+                              ctl.busy_cycles, ctl.idle_cycles, ctl.pieces,
+                              ctl.steps,       ctl.lanes};
+  memcpy(needs_out, needs, sizeof(needs));
 }
 
 static bool caps_ok(const TwCaps& c) {
@@ -1522,21 +1674,7 @@ int ygx_target_walk(const float* center, const float* radius, const float* max_e
     return YGX_ERR_CUDA;
   const int32_t T = (int32_t)total, NI = (int32_t)num_internal;
   const float th = theta;
-  // allocation blocks: small enough that every warp's open blocks fit the
-  // pools many times over, large enough to keep the global cursors quiet
-  unsigned long long blk_entries;
-  unsigned blk_records;
-  {
-    const long long nwarps = (long long)kNumSMs * kTwBlocksPerSM * kTwWarps;
-    long long me = c.far < c.near_ ? c.far : c.near_;
-    me = me < c.split ? me : c.split;
-    long long be = me / (nwarps * 16);
-    blk_entries = (unsigned long long)(be < 32 ? 32 : (be > 2048 ? 2048 : be));
-    long long mr = c.far_rec < c.near_rec ? c.far_rec : c.near_rec;
-    mr = mr < c.s_rec ? mr : c.s_rec;
-    long long br = mr / (nwarps * 8);
-    blk_records = (unsigned)(br < 4 ? 4 : (br > 64 ? 64 : br));
-  }
+  const TwBlocks blk(c);
   cudaError_t e = cudaSuccess;
   if (pairs) {
     k_pw_slots<<<grid_for(total, 256), 256, 0, stream>>>(
@@ -1544,65 +1682,14 @@ int ygx_target_walk(const float* center, const float* radius, const float* max_e
         s.sid, s.queue32, s.q_ready, s.ctl, leafpos32, far_rcap32, near_rcap32, pad_far, pad_near,
         s.pw_rows, s.first_ovf_far, s.first_ovf_near, s.status);
     YGX_CHECK_LAUNCH();
-    PwArgs a;
-    a.sc = s.sc;
-    a.sid = s.sid;
+    PwArgs a = pair_args(s, c, T - 1, th);
     a.rows = s.pw_rows;
-    a.ni = NI;
-    a.n_targets = T - 1;
-    a.theta_sq = th * th;
-    a.theta = sqrtf(a.theta_sq);
-    a.s_cnt = s.s_cnt;
-    a.s_nch = s.s_nch;
-    a.s_head = s.s_head;
-    a.pieces_left = s.pieces_left;
-    a.far_cnt = s.far_cnt;
-    a.near_cnt = s.near_cnt;
-    a.far_pool = s.far_pool;
-    a.near_pool = s.near_pool;
-    a.s_pool = s.s_pool32;
-    a.spill = s.spill32;
-    a.far_cap = (unsigned long long)c.far;
-    a.near_cap = (unsigned long long)c.near_;
-    a.s_cap = (unsigned long long)c.split;
-    a.spill_cap = (unsigned long long)c.spill;
-    a.far_keys = s.far_keys;
-    a.far_recs = s.far_recs;
-    a.near_keys = s.near_keys;
-    a.near_recs = s.near_recs;
-    a.s_recs = s.s_recs;
-    a.far_rec_cap = (unsigned)c.far_rec;
-    a.near_rec_cap = (unsigned)c.near_rec;
-    a.s_rec_cap = (unsigned)c.s_rec;
-    a.q_cap = (unsigned)c.queue;
-    a.queue = s.queue32;
-    a.q_ready = s.q_ready;
-    a.gen_hist = s.gen_hist;
-    a.ctl = s.ctl;
-    a.status = s.status;
-    a.spin_limit = (uint32_t)g_tune.spin_limit;
-    a.budget = g_tune.target_budget;
-    a.blk_entries = blk_entries;
-    a.blk_records = blk_records;
+    a.near_rows = s.pw_rows + L;  // leaf node num_internal + j at total + j
     a.far_raw = far_raw;
     a.near_raw = near_raw;
     a.first_ovf_far = pred ? s.first_ovf_far : nullptr;
     a.first_ovf_near = pred ? s.first_ovf_near : nullptr;
-    const size_t smem = sizeof(PwSmem);
-    static std::atomic<uint64_t> attr[3];
-    // a small tree never has work for every warp of the device; fewer CTAs
-    // start and end sooner
-    const int grid = grid_for(total, 16, kNumSMs * kPwBlocksPerSM);
-    a.hungry = grid * kPwWarps / 4;
-#define YGX_PW(M)                                                                    \
-  e = ensure_smem_limit(k_pair_walk<M>, (int)smem, attr[M]);                         \
-  if (e == cudaSuccess) k_pair_walk<M><<<grid, kPwThreads, smem, stream>>>(a)
-    switch (mac) {
-      case kTwBH: YGX_PW(kTwBH); break;
-      case kTwDehnen: YGX_PW(kTwDehnen); break;
-      default: YGX_PW(kTwEngblom); break;
-    }
-#undef YGX_PW
+    e = launch_pair_walk(a, mac, total, stream);
   } else {
     k_tw_first_leaf<<<grid_for(L, 256), 256, 0, stream>>>(parent32, left32, NI, T, s.first);
     YGX_CHECK_LAUNCH();
@@ -1666,8 +1753,8 @@ int ygx_target_walk(const float* center, const float* radius, const float* max_e
     a.near_raw = near_raw;
     a.first_ovf_far = pred ? s.first_ovf_far : nullptr;
     a.first_ovf_near = pred ? s.first_ovf_near : nullptr;
-    a.blk_entries = blk_entries;
-    a.blk_records = blk_records;
+    a.blk_entries = blk.entries;
+    a.blk_records = blk.records;
     const size_t smem = sizeof(TwSmem);
     static std::atomic<uint64_t> attr[6];
     const int grid = kNumSMs * kTwBlocksPerSM;
@@ -1696,75 +1783,77 @@ int ygx_target_walk(const float* center, const float* radius, const float* max_e
       pred ? near_rcap32 : nullptr, tree_level_offsets, index_bits, num_levels, s.levels,
       s.rowstat);
   YGX_CHECK_LAUNCH();
-  // status word, control block, histogram, row statistics and levels lie one
-  // behind the other: one read
-  alignas(16) char block[8192];
-  const char* first = (const char*)s.status;
-  const size_t bytes = (const char*)(s.levels + kTwHist / 2 + 1) - first;
-  if (bytes > sizeof(block)) return YGX_ERR_ARG;
-  if (cudaMemcpyAsync(block, first, bytes, cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
-      cudaStreamSynchronize(stream) != cudaSuccess)
+  TwRead r;
+  const int rc = read_walk(s, &r, stream);
+  if (rc) return rc;
+  flags_out[0] = r.flags;
+  int64_t level_count[kTwHist / 2];
+  for (int l = 0; l < num_levels; ++l) level_count[l] = r.levels[l + 1] - r.levels[l];
+  walk_stats(r, level_count, num_levels, total, pred, stats_out, needs_out);
+  return YGX_OK;
+}
+
+// The forest of batched sets through the pair walk (see ygx.h).
+size_t ygx_batch_target_walk_workspace_size(int64_t total, int64_t num_leaves,
+                                            const int64_t* caps) {
+  if (!caps) return 0;
+  ygx::TwCaps c{caps[0], caps[1], caps[2], caps[3], caps[4], caps[5], caps[6], caps[7]};
+  ygx::Arena a{nullptr, 0, 0};
+  ygx::carve_tw(a, total, num_leaves, c, false, true);
+  return a.used + 256;
+}
+
+int ygx_batch_target_walk(const float* center, const float* radius, const float* max_extent,
+                          const int32_t* left32, const int32_t* right32,
+                          const int32_t* leafpos32, const int32_t* level32, int64_t total,
+                          int64_t num_leaves, const int64_t* leaf_off, int64_t S,
+                          const uint32_t* seg_flags, int mac, float theta,
+                          float dehnen_radius_scale, const int64_t* caps, uint64_t* stats_out,
+                          uint64_t* needs_out, uint32_t* flags_out, void* ws, size_t ws_bytes,
+                          cudaStream_t stream) {
+  using namespace ygx;
+  if (total < 3 || 2 * total > kPwMaxNodes || num_leaves < 2 || S < 1 ||
+      total != 2 * num_leaves - S || mac < 0 || mac > 2 || !caps || !stats_out || !needs_out ||
+      !flags_out || !center || !radius || !max_extent || !left32 || !right32 || !leafpos32 ||
+      !level32 || !leaf_off || !seg_flags || !ws)
+    return YGX_ERR_ARG;
+  TwCaps c{caps[0], caps[1], caps[2], caps[3], caps[4], caps[5], caps[6], caps[7]};
+  if (!caps_ok(c) || ws_bytes < ygx_batch_target_walk_workspace_size(total, num_leaves, caps))
+    return YGX_ERR_ARG;
+  Arena ar{(char*)ws, 0, ws_bytes};
+  TwScratch s = carve_tw(ar, total, num_leaves, c, false, true);
+  if (cudaMemsetAsync(s.status, 0, (size_t)((char*)(s.q_ready + c.queue) - (char*)s.status),
+                      stream) != cudaSuccess)
     return YGX_ERR_CUDA;
-  auto at = [&](const void* p) { return block + ((const char*)p - first); };
-  TwCtl ctl;
-  unsigned int hist[kTwHist];
-  unsigned long long rs[8];
-  int64_t lvl_off[kTwHist / 2 + 1];
-  memcpy(flags_out, at(s.status), sizeof(uint32_t));
-  memcpy(&ctl, at(s.ctl), sizeof(ctl));
-  memcpy(hist, at(s.gen_hist), sizeof(hist));
-  memcpy(rs, at(s.rowstat), sizeof(rs));
-  memcpy(lvl_off, at(s.levels), sizeof(int64_t) * (num_levels + 1));
-  // generations: every node's self pair {v, v} sits at generation depth(v);
-  // every other pair was evaluated once from each side
-  unsigned long long wf2[kTwHist];
-  for (int g = 0; g < kTwHist; ++g) wf2[g] = hist[g];
-  for (int l = 0; l < num_levels && l < kTwHist; ++l)
-    wf2[l] += 2ull * (unsigned long long)(lvl_off[l + 1] - lvl_off[l]);
-  unsigned long long mw = 1, gens = 0;
-  for (int g = 0; g < kTwHist; ++g) {
-    if (wf2[g] == 0) continue;
-    gens = (unsigned long long)g + 1;
-    if (g > 0 && wf2[g] / 2 > mw) mw = wf2[g] / 2;
-  }
-  for (int k = 0; k < YGX_TSTAT_WORDS; ++k) stats_out[k] = 0;
-  stats_out[YGX_TSTAT_FAR_TOTAL] = rs[0];
-  stats_out[YGX_TSTAT_NEAR_TOTAL] = rs[1];
-  stats_out[YGX_TSTAT_MAX_FAR] = rs[2];
-  stats_out[YGX_TSTAT_MAX_NEAR] = rs[3];
-  stats_out[YGX_TSTAT_ACCEPT] = ctl.acc_sides / 2;
-  stats_out[YGX_TSTAT_NEAR] = ctl.near_sides / 2;
-  stats_out[YGX_TSTAT_REFINE] = ctl.ref_sides / 2 + (unsigned long long)total;
-  stats_out[YGX_TSTAT_MAX_WF] = mw;
-  stats_out[YGX_TSTAT_GENS] = gens;
-  if (pred) {
-    stats_out[YGX_TSTAT_OVF_ROWS] = rs[4];
-    stats_out[YGX_TSTAT_OVF_ENTRIES] = rs[5];
-    stats_out[YGX_TSTAT_EXT_FAR] = rs[6];
-    stats_out[YGX_TSTAT_EXT_NEAR] = rs[7];
-  }
-  // what each capacity needed (a re-run with these fits)
-  needs_out[0] = ctl.far_cur;
-  needs_out[1] = ctl.near_cur;
-  needs_out[2] = ctl.s_cur;
-  needs_out[3] = ctl.spill_cur;
-  needs_out[4] = ctl.far_rec_cur;
-  needs_out[5] = ctl.near_rec_cur;
-  needs_out[6] = ctl.s_rec_cur;
-  needs_out[7] = ctl.q_tail;
-  needs_out[8] = ctl.max_cmp;
-  needs_out[9] = ctl.busy_cycles;  // warp cycles on pieces / waiting, pieces run
-  needs_out[10] = ctl.idle_cycles;
-  needs_out[11] = ctl.pieces;
-  needs_out[12] = ctl.steps;  // 32-wide steps and the candidates they held
-  needs_out[13] = ctl.lanes;
+  const int32_t T = (int32_t)total;
+  k_pw_forest_slots<<<grid_for(total > S ? total : S, 256, kNumSMs * 8), 256, 0, stream>>>(
+      center, radius, max_extent, left32, right32, leafpos32, level32, T, leaf_off, S, seg_flags,
+      mac, dehnen_radius_scale, s.sc, s.sid, s.queue32, s.q_ready, (unsigned)c.queue, s.ctl,
+      s.pw_rows, s.pw_rows + total, s.levels, s.status);
+  YGX_CHECK_LAUNCH();
+  PwArgs a = pair_args(s, c, (int32_t)(total - S), theta);
+  a.rows = s.pw_rows;
+  a.near_rows = s.pw_rows + total;
+  if (launch_pair_walk(a, mac, total, stream) != cudaSuccess) return YGX_ERR_CUDA;
+  YGX_CHECK_LAUNCH();
+  k_tw_row_stats<<<grid_for(total, 256, kNumSMs * 4), 256, 0, stream>>>(
+      s.far_cnt, T, s.near_cnt, (int32_t)num_leaves, nullptr, nullptr, nullptr, 64, -1, s.levels,
+      s.rowstat);
+  YGX_CHECK_LAUNCH();
+  TwRead r;
+  const int rc = read_walk(s, &r, stream);
+  if (rc) return rc;
+  flags_out[0] = r.flags;
+  walk_stats(r, r.levels, kTwHist / 2, total, false, stats_out, needs_out);
   return YGX_OK;
 }
 
 // After ygx_target_walk on the same workspace (and with its capacities):
 // the level-major far lists and the leaf-order near lists in the index dtype,
-// with the reference's offset / count tables.
-int ygx_target_walk_lists(int64_t total, int64_t num_internal, const int64_t* caps, int ordered,
+// with the reference's offset / count tables.  far_base / near_base: per row
+// the id to subtract from every id written (a forest's local ids), or null.
+static int walk_lists(bool forest, const int32_t* far_row_base, const int32_t* near_row_base,
+                      int64_t total, int64_t num_internal, const int64_t* caps, int ordered,
                           const int32_t* far_rcap32, const int32_t* near_rcap32,
                           const int64_t* pad_far, const int64_t* pad_near, int32_t* far_raw,
                           int64_t far_raw_cap, int32_t* near_raw, int64_t near_raw_cap,
@@ -1782,7 +1871,9 @@ int ygx_target_walk_lists(int64_t total, int64_t num_internal, const int64_t* ca
     return YGX_ERR_ARG;
   TwCaps c{caps[0], caps[1], caps[2], caps[3], caps[4], caps[5], caps[6], caps[7]};
   if (!caps_ok(c)) return YGX_ERR_ARG;
-  if (ws_bytes < ygx_target_walk_workspace_size(total, total - num_internal, caps, ordered))
+  const int64_t L = total - num_internal;
+  if (ws_bytes < (forest ? ygx_batch_target_walk_workspace_size(total, L, caps)
+                         : ygx_target_walk_workspace_size(total, L, caps, ordered)))
     return YGX_ERR_ARG;
   if ((int64_t)far_records > c.far_rec || (int64_t)near_records > c.near_rec) return YGX_ERR_ARG;
   const bool pred = far_rcap32 != nullptr;
@@ -1791,9 +1882,8 @@ int ygx_target_walk_lists(int64_t total, int64_t num_internal, const int64_t* ca
   if (pred && (!near_rcap32 || !pad_far || !pad_near)) return YGX_ERR_ARG;
   if (!ordered && !pred && (far_total > far_raw_cap || near_total > near_raw_cap))
     return YGX_ERR_ARG;
-  const int64_t L = total - num_internal;
   Arena ar{(char*)ws, 0, ws_bytes};
-  TwScratch s = carve_tw(ar, total, L, c, ordered != 0);
+  TwScratch s = carve_tw(ar, total, L, c, ordered != 0, forest);
   const int32_t T = (int32_t)total;
   // offset / count tables and where the raw rows sit
   const TwPlan plan{s.far_cnt,  s.near_cnt,   far_rcap32,   near_rcap32,  nbl32,
@@ -1833,10 +1923,11 @@ int ygx_target_walk_lists(int64_t total, int64_t num_internal, const int64_t* ca
       YGX_CHECK_LAUNCH();
     }
     const RowTable far_rows{total, s.far_off_node, s.far_cnt, level32, far_raw,
-                            pred ? s.roff_far : nullptr, nullptr, sources, targets,
+                            pred ? s.roff_far : nullptr, far_row_base, sources, targets,
                             target_levels};
     const RowTable near_rows{L, s.near_off, s.near_cnt, nullptr, near_raw,
-                             pred ? s.roff_near : nullptr, nullptr, neighbors, nullptr, nullptr};
+                             pred ? s.roff_near : nullptr, near_row_base, neighbors, nullptr,
+                             nullptr};
     rc = row_sort_pass(s.rs, far_rows, near_rows, index_bits, total, stream);
     if (rc) return rc;
   } else {
@@ -1878,6 +1969,46 @@ int ygx_target_walk_lists(int64_t total, int64_t num_internal, const int64_t* ca
     YGX_CHECK_LAUNCH();
   }
   return YGX_OK;
+}
+
+int ygx_target_walk_lists(int64_t total, int64_t num_internal, const int64_t* caps, int ordered,
+                          const int32_t* far_rcap32, const int32_t* near_rcap32,
+                          const int64_t* pad_far, const int64_t* pad_near, int32_t* far_raw,
+                          int64_t far_raw_cap, int32_t* near_raw, int64_t near_raw_cap,
+                          const int32_t* nbl32, const int32_t* level32,
+                          const void* tree_level_offsets, int num_levels, int index_bits,
+                          int64_t far_total, int64_t near_total, uint64_t far_records,
+                          uint64_t near_records, void* node_offsets, void* far_counts,
+                          void* level_offsets, void* sources, void* targets, void* target_levels,
+                          void* near_offsets, void* near_counts, void* neighbors,
+                          const int32_t* leafpos32, int64_t max_nbr,
+                          void* neighbor_leaf_positions, void* ws, size_t ws_bytes,
+                          cudaStream_t stream) {
+  return walk_lists(false, nullptr, nullptr, total, num_internal, caps, ordered, far_rcap32,
+                    near_rcap32, pad_far, pad_near, far_raw, far_raw_cap, near_raw, near_raw_cap,
+                    nbl32, level32, tree_level_offsets, num_levels, index_bits, far_total,
+                    near_total, far_records, near_records, node_offsets, far_counts,
+                    level_offsets, sources, targets, target_levels, near_offsets, near_counts,
+                    neighbors, leafpos32, max_nbr, neighbor_leaf_positions, ws, ws_bytes, stream);
+}
+
+int ygx_batch_target_walk_lists(int64_t total, int64_t num_leaves, const int64_t* caps,
+                                int32_t* far_raw, int64_t far_raw_cap, int32_t* near_raw,
+                                int64_t near_raw_cap, const int32_t* nbl32,
+                                const int32_t* level32, const int32_t* far_row_base,
+                                const int32_t* near_row_base, int index_bits, int64_t far_total,
+                                int64_t near_total, uint64_t far_records, uint64_t near_records,
+                                void* node_offsets, void* far_counts, void* sources,
+                                void* targets, void* target_levels, void* near_offsets,
+                                void* near_counts, void* neighbors, void* ws, size_t ws_bytes,
+                                cudaStream_t stream) {
+  if (2 * total > ygx::kPwMaxNodes) return YGX_ERR_ARG;
+  return walk_lists(true, far_row_base, near_row_base, total, total - num_leaves, caps, 0, nullptr,
+                    nullptr, nullptr, nullptr, far_raw, far_raw_cap, near_raw, near_raw_cap, nbl32,
+                    level32, nullptr, -1, index_bits, far_total, near_total, far_records,
+                    near_records, node_offsets, far_counts, nullptr, sources, targets,
+                    target_levels, near_offsets, near_counts, neighbors, nullptr, 0, nullptr, ws,
+                    ws_bytes, stream);
 }
 
 // Padded row slots for predicted capacities: pad_far[0..total] and

@@ -522,6 +522,16 @@ def _target_caps(total: int, nl: int, hint) -> list:
             4 * nl + near // 32 + 4096, 4 * total + split // 64 + 4096, 4 * total + 65536]
 
 
+def _grow_target_caps(caps: list, needs, runs: int, flags: int) -> list:
+    """Capacities for the re-run of a target walk that overflowed.  A walk cut
+    short by one capacity reports only the needs of the work it did: grow
+    what overflowed by 2x its need."""
+    grown = [c if int(n) <= c else 2 * int(n) + 4096 for c, n in zip(caps, needs[:8])]
+    if grown == caps or runs > 12:
+        raise L.YgxError(f"target walk capacities did not converge (flags {flags:#x})")
+    return grown
+
+
 def _target_walk(topology, d, total, ni, nl, num_levels, center, radius, max_extent, leafpos32,
                  theta, mac_type, mac, dehnen_radius_scale, root, timing, evs, ordered,
                  learned=False):
@@ -595,12 +605,7 @@ def _target_walk(topology, d, total, ni, nl, num_levels, center, radius, max_ext
                                "log schedule", f)
             return None
         if f & L.FLAG_LOG_OVERFLOW:
-            # A walk cut short by one capacity reports only the needs of the
-            # work it did: grow what overflowed by 2x its need and re-run.
-            grown = [c if int(n) <= c else 2 * int(n) + 4096 for c, n in zip(caps, needs[:8])]
-            if grown == caps or runs > 12:
-                raise L.YgxError(f"target walk capacities did not converge (flags {f:#x})")
-            caps = grown
+            caps = _grow_target_caps(caps, needs, runs, f)
             ws = far_raw = near_raw = None
             continue
         if f:
