@@ -8,11 +8,10 @@
 namespace ygx {
 
 struct RowSortScratch {
-  uint32_t* n_big;      // 64 words: long-row and class counters
-  int32_t* big_rows;    // stride entries
-  int32_t* class_rows;  // one list of stride rows per size class
-  uint32_t* bitmaps;    // one bitmap over [0, universe) per long-row CTA
-  int64_t stride;       // rows of both tables of a pass together
+  uint32_t* counts;   // 64 words: rows per size class, the long rows' work counter
+  int32_t* lists;     // lists of stride rows, one per two size classes
+  uint32_t* bitmaps;  // one bitmap over [0, universe) per long-row CTA
+  int64_t stride;     // rows of both tables of a pass together
 };
 
 // One list's rows: row r has cnt[r] raw int32 values at raw + (roff ?
@@ -37,9 +36,8 @@ struct RowTable {
 RowSortScratch carve_row_sort(Arena& a, int64_t total, int64_t L);
 
 // Sorts the rows of both tables in one pass (b.rows may be 0): one size
-// classification, one launch per size class and one long-row launch for
-// both, so the longest rows of either start first and the rest fill in
-// around them.  Does not synchronize.
+// classification and one launch per kind of row (long, several warps, one
+// warp) for both.  Does not synchronize.
 int row_sort_pass(const RowSortScratch& s, const RowTable& a, const RowTable& b, int index_bits,
                   int64_t universe, cudaStream_t stream);
 

@@ -1450,7 +1450,7 @@ static TwScratch carve_tw(Arena& a, int64_t total, int64_t L, const TwCaps& c, b
   s.far_off_node = nullptr;
   s.first_ovf_far = s.first_ovf_near = nullptr;
   s.ext_far = s.ext_near = s.roff_far = s.roff_near = nullptr;
-  s.rs = RowSortScratch{nullptr, nullptr, nullptr, nullptr, 0};
+  s.rs = RowSortScratch{nullptr, nullptr, nullptr, 0};
   if (!ordered) {
     s.far_off_node = a.take<int64_t>(total + 1);
     s.first_ovf_far = a.take<unsigned>(total);

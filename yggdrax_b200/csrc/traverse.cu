@@ -19,6 +19,7 @@
 // endpoints' rows at atomic cursors; the finalize pass sorts every row
 // (canonical order) and widens it into the level-major int64/int32 outputs.
 #include "rows.cuh"
+#include "row_sort.cuh"
 #include "scan.cuh"
 
 namespace ygx {
@@ -773,19 +774,17 @@ __global__ void k_near_offsets(const int64_t* __restrict__ off, const int32_t* _
 }
 
 // ---------------------------------------------------------------------------
-// Row finalize: sort each row ascending and widen it.  The network is the
-// all-ascending ("mirrored") bitonic sort: for each block size k the first
-// step pairs i with i ^ (k - 1), later steps pair i with i ^ j.  Every
-// comparator puts the minimum at the lower index, so a row of any length n
-// sorts as if padded with +inf, and comparators whose upper index is >= n
-// are no-ops that can be skipped -- no padding storage is needed.
-// Rows up to kWarpRowCap entries: one warp in shared memory; up to
-// kBlockRowCap: one CTA in shared memory; longer: one CTA in place in
-// global memory.
+// Row finalize of long rows (shorter ones: row_sort.cuh).  Rows the bitmap
+// cannot order go through the all-ascending ("mirrored") bitonic sort: for
+// each block size k the first step pairs i with i ^ (k - 1), later steps pair
+// i with i ^ j.  Every comparator puts the minimum at the lower index, so a
+// row of any length n sorts as if padded with +inf, and comparators whose
+// upper index is >= n are no-ops that can be skipped -- no padding storage is
+// needed.  Up to kBlockRowCap entries in shared memory, longer rows in place
+// in global memory.
 
-constexpr int kWarpRowCap = 1024;   // one warp, 4 KB of shared memory
 constexpr int kBlockRowCap = 16384; // one CTA, 64 KB of shared memory
-constexpr int kBigThreads = 512;
+constexpr int kBigThreads = kCtaThreads;
 
 template <bool kBlockSync>
 __device__ __forceinline__ void mirrored_bitonic(int32_t* a, int64_t n64, int tid, int nthreads) {
@@ -824,156 +823,6 @@ __device__ __forceinline__ void emit_row(const int32_t* a, int64_t n, int64_t of
       store_idx(tgt_out, index_bits, off + k, tgt);
       store_idx(lvl_out, index_bits, off + k, lvl);
     }
-  }
-}
-
-// One warp sorts a row of up to 32*R entries held in registers in the
-// "blocked" layout: lane l holds elements l*R .. l*R+R-1.  Loads and stores
-// stay coalesced through a padded shared-memory transpose (row stride R+1,
-// conflict-free both ways).  With this layout the bitonic steps with
-// partner distance j < R are compare-exchanges between registers of one
-// lane and only the steps with j >= R exchange across lanes (shuffles).
-// The row is padded with INT32_MAX to 32*R entries.
-template <int R>
-__device__ __forceinline__ void warp_sort_row(const int32_t* __restrict__ raw, int64_t roff,
-                                              int64_t off,
-                                              int n, int index_bits, void* vals_out,
-                                              void* tgt_out, void* lvl_out, int32_t tgt,
-                                              int32_t vbase, int32_t lvl, int lane,
-                                              int32_t* __restrict__ sm) {
-  constexpr int S = R + 1;
-  constexpr int LOGR = R == 1 ? 0 : R == 2 ? 1 : R == 4 ? 2 : R == 8 ? 3 : R == 16 ? 4 : 5;
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int e = r * 32 + lane;
-    sm[(e >> LOGR) * S + (e & (R - 1))] = e < n ? raw[roff + e] : INT32_MAX;
-  }
-  __syncwarp();
-  int32_t v[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) v[r] = sm[lane * S + r];
-  // All-ascending network: every comparator puts the minimum at the lower
-  // index, so no per-comparator direction is needed.  The first step of a
-  // k-block pairs i with i ^ (k - 1): inside a lane register r with r ^
-  // (k - 1) while k <= R, else lane l ^ (k / R - 1), register R - 1 - r.
-#pragma unroll
-  for (int k = 2; k <= 32 * R; k <<= 1) {
-    if (k <= R) {
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int rp = r ^ (k - 1);
-        if (rp > r) {
-          const int32_t x = v[r], y = v[rp];
-          v[r] = min(x, y);
-          v[rp] = max(x, y);
-        }
-      }
-    } else {
-      const int m = (k >> LOGR) - 1;
-      const bool lower = (lane & ((k >> LOGR) >> 1)) == 0;
-      int32_t y[R];
-#pragma unroll
-      for (int r = 0; r < R; ++r) y[r] = __shfl_xor_sync(0xffffffffu, v[R - 1 - r], m);
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = lower ? min(v[r], y[r]) : max(v[r], y[r]);
-    }
-#pragma unroll
-    for (int j = k >> 2; j > 0; j >>= 1) {
-      if (j < R) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          if ((r & j) == 0) {
-            const int rp = r | j;
-            const int32_t x = v[r], y = v[rp];
-            v[r] = min(x, y);
-            v[rp] = max(x, y);
-          }
-        }
-      } else {
-        const int lj = j >> LOGR;
-        const bool lower = (lane & lj) == 0;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int32_t y = __shfl_xor_sync(0xffffffffu, v[r], lj);
-          v[r] = lower ? min(v[r], y) : max(v[r], y);
-        }
-      }
-    }
-  }
-  __syncwarp();
-#pragma unroll
-  for (int r = 0; r < R; ++r) sm[lane * S + r] = v[r];
-  __syncwarp();
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int e = r * 32 + lane;
-    if (e < n) {
-      const int32_t x = sm[(e >> LOGR) * S + (e & (R - 1))];
-      store_idx(vals_out, index_bits, off + e, x - vbase);
-      if (tgt_out) {
-        store_idx(tgt_out, index_bits, off + e, tgt);
-        store_idx(lvl_out, index_bits, off + e, lvl);
-      }
-    }
-  }
-  __syncwarp();
-}
-
-// Rows are bucketed by size class first; each class runs in its own kernel
-// with a single register-network instantiation (one instantiation per
-// kernel keeps the instruction footprint small).  Class c holds rows of
-// 32*2^(c-1) < n <= 32*2^c entries (c = 0: n <= 32); longer rows go to the
-// CTA kernel.
-constexpr int kRowClasses = 6;  // R = 1, 2, 4, 8, 16, 32
-
-// Rows of two tables in one pass: row r < ta.rows is ta's row r, the others
-// are tb's row r - ta.rows.
-__global__ void k_rows_classify(RowTable ta, RowTable tb, int32_t* __restrict__ lists,
-                                int64_t list_stride, uint32_t* __restrict__ list_n,
-                                int32_t* __restrict__ big_rows, uint32_t* __restrict__ n_big) {
-  const int64_t rows = ta.rows + tb.rows;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows;
-       r += (int64_t)gridDim.x * blockDim.x) {
-    const int n = r < ta.rows ? ta.cnt[r] : tb.cnt[r - ta.rows];
-    if (n == 0) continue;
-    if (n > kWarpRowCap) {
-      // rows longer than kBlockRowCap from the front, the others from the
-      // back: the long-row kernel takes the longest first
-      if (n > kBlockRowCap) big_rows[atomicAdd(&n_big[0], 1u)] = (int32_t)r;
-      else big_rows[list_stride - 1 - atomicAdd(&n_big[8], 1u)] = (int32_t)r;
-      continue;
-    }
-    int c = 0;
-    while ((32 << c) < n) ++c;
-    // warp-aggregated append per class
-    const unsigned m = __activemask();
-    const unsigned peers = __match_any_sync(m, c);
-    const int leader = __ffs(peers) - 1;
-    uint32_t base = 0;
-    if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(&list_n[c], (uint32_t)__popc(peers));
-    base = __shfl_sync(peers, base, leader);
-    unsigned lt;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-    lists[c * list_stride + base + __popc(peers & lt)] = (int32_t)r;
-  }
-}
-
-template <int R>
-__global__ void __launch_bounds__(256, R >= 32 ? 2 : (R >= 16 ? 3 : 4))
-    k_rows_class(const int32_t* __restrict__ list, const uint32_t* __restrict__ list_n,
-                 RowTable ta, RowTable tb, int index_bits) {
-  __shared__ int32_t s_rows[8][32 * (R + 1)];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint32_t nm = *list_n;
-  for (uint32_t b = blockIdx.x * 8 + w; b < nm; b += gridDim.x * 8) {
-    const int32_t g = list[b];
-    const bool second = g >= ta.rows;
-    const RowTable& T = second ? tb : ta;
-    const int32_t r = second ? g - (int32_t)ta.rows : g;
-    const int32_t vbase = T.rbase ? T.rbase[r] : 0;
-    warp_sort_row<R>(T.raw, T.roff ? T.roff[r] : T.off[r], T.off[r], T.cnt[r], index_bits,
-                     T.vals, T.tgts, T.lvls, r - vbase, vbase, T.lvl ? T.lvl[r] : 0, lane,
-                     s_rows[w]);
   }
 }
 
@@ -1016,8 +865,8 @@ __device__ __forceinline__ int64_t block_excl_scan(int64_t v, int64_t* s_tmp, in
   return wpre + incl - v;
 }
 
-// Long rows (> kWarpRowCap entries): one CTA per row, rows taken from a
-// work counter longest first.  A row holds distinct node ids (a canonical
+// Long rows (> kCtaRowCap entries): one CTA per row, rows taken from a
+// work counter, the longest classes first.  A row holds distinct node ids (a canonical
 // pair is visited once), so it is ordered through a two-level bitmap over
 // its value range [min, max]: one bit per value (in shared memory when the
 // range fits kBlockRowCap words, else in this CTA's global bitmap) and one
@@ -1029,9 +878,10 @@ __device__ __forceinline__ int64_t block_excl_scan(int64_t v, int64_t* s_tmp, in
 // are cleared again.  Repeated entries (seen when a bit was already set) or
 // ranges beyond the summary send the row to a bitonic network instead (in
 // shared memory up to kBlockRowCap entries, else in place in global memory).
-__global__ void __launch_bounds__(kBigThreads, 3)
-    k_rows_big(const int32_t* __restrict__ big_rows, uint32_t* __restrict__ n_big,
-               int64_t list_cap, RowTable ta, RowTable tb, int index_bits,
+template <typename Idx>
+__global__ void __launch_bounds__(kBigThreads, 1)
+    k_rows_big(const int32_t* __restrict__ lists, int64_t stride, uint32_t* __restrict__ counts,
+               RowTable ta, RowTable tb,
                uint32_t* __restrict__ bitmaps, int64_t universe) {
   extern __shared__ uint32_t s_dyn[];  // kBlockRowCap words: bitmap, or a row to sort
   __shared__ uint32_t s_sum[kSumWords];
@@ -1040,25 +890,33 @@ __global__ void __launch_bounds__(kBigThreads, 3)
   __shared__ int32_t s_min[32], s_max[32];
   __shared__ uint32_t s_item;
   __shared__ int s_dup;
-  const uint32_t n_long = n_big[0], n_mid = n_big[8];
+  uint32_t n_long = 0;
+  for (int c = 0; c < kLongClasses; ++c) n_long += counts[kRowClasses - 1 - c];
+  __shared__ uint32_t s_next[kBigThreads / 128];
+  const bool any_long = blockIdx.x < n_long;  // else straight to the shorter rows
+  constexpr int index_bits = 8 * sizeof(Idx);
   const int64_t gwords = (universe + 31) / 32;
   uint32_t* gbm = bitmaps + (int64_t)blockIdx.x * gwords;
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
   const int nwarps = nt >> 5;
-  for (int w = tid; w < kBlockRowCap; w += nt) s_dyn[w] = 0u;
+  if (any_long)
+    for (int w = tid; w < kBlockRowCap; w += nt) s_dyn[w] = 0u;
   for (int w = tid; w < kSumWords; w += nt) s_sum[w] = 0u;
-  if (gwords > kBlockRowCap)
+  if (any_long && gwords > kBlockRowCap)
     for (int64_t w = tid; w < gwords; w += nt) gbm[w] = 0u;
   __syncthreads();
   __shared__ RowTable s_tab;  // the current row's table (picked by thread 0)
   __shared__ int32_t s_row;
-  while (true) {
+  while (any_long) {
     if (tid == 0) {
-      const uint32_t bb = atomicAdd(&n_big[9], 1u);
+      const uint32_t bb = atomicAdd(&counts[kRowWork], 1u);
       s_item = bb;
       s_dup = 0;
-      if (bb < n_long + n_mid) {
-        const int32_t g = bb < n_long ? big_rows[bb] : big_rows[list_cap - 1 - (bb - n_long)];
+      if (bb < n_long) {
+        uint32_t k = bb;
+        int c = kRowClasses - 1;
+        while (k >= counts[c]) k -= counts[c--];
+        const int32_t g = lists[row_slot(c, k, stride)];
         const bool second = g >= ta.rows;
         s_tab = second ? tb : ta;
         s_row = second ? g - (int32_t)ta.rows : g;
@@ -1066,7 +924,7 @@ __global__ void __launch_bounds__(kBigThreads, 3)
     }
     __syncthreads();
     const uint32_t b = s_item;
-    if (b >= n_long + n_mid) break;
+    if (b >= n_long) break;
     const RowTable& T = s_tab;
     const int32_t r = s_row;
     const int64_t* __restrict__ row_off = T.off;
@@ -1291,6 +1149,7 @@ __global__ void __launch_bounds__(kBigThreads, 3)
     }
     __syncthreads();
   }
+  sort_cta_rows<Idx>(ta, tb, lists, stride, counts, reinterpret_cast<int32_t*>(s_dyn), s_next);
 }
 
 // Dense neighbour leaf positions (L x max_nbr) of _result_to_neighbors.
@@ -1326,8 +1185,7 @@ struct TravScratch {
   unsigned long long* far_pos;
   unsigned long long* near_pos;
   int64_t* scan_tmp;
-  int32_t* big_rows;
-  int32_t* class_rows;  // kRowClasses lists of total + L rows
+  int32_t* row_lists;  // kRowLists lists of total + L rows
   uint32_t* bitmaps;
   int2* wf[2];
   uint32_t* region_cnt[2];
@@ -1357,41 +1215,51 @@ static int64_t region_capacity(int64_t cap) {
   const int64_t r = cap / kWalkGrid;
   return r < kMinRegion ? kMinRegion : r;
 }
-constexpr int kBigGrid = kNumSMs * 3;
+constexpr int kBigGrid = kNumSMs;
 
 RowSortScratch carve_row_sort(Arena& a, int64_t total, int64_t L) {
   RowSortScratch s;
   s.stride = total + L;
-  s.n_big = a.take<uint32_t>(64);
-  s.big_rows = a.take<int32_t>(s.stride);
-  s.class_rows = a.take<int32_t>((size_t)kRowClasses * s.stride);
+  s.counts = a.take<uint32_t>(64);
+  s.lists = a.take<int32_t>((size_t)kRowLists * s.stride);
   s.bitmaps = a.take<uint32_t>((size_t)kBigGrid * ((total + 31) / 32));
   return s;
 }
 
-int row_sort_pass(const RowSortScratch& s, const RowTable& a, const RowTable& b, int index_bits,
-                  int64_t universe, cudaStream_t stream) {
-  const int grid_small = kNumSMs * g_tune.row_grid_per_sm;
-  const size_t big_smem = sizeof(int32_t) * kBlockRowCap;
+template <typename Idx>
+static int row_sort_launch(const RowSortScratch& s, const RowTable& a, const RowTable& b,
+                           int64_t universe, cudaStream_t stream) {
+  constexpr int kWords = kBlockRowCap > kCtaWords ? kBlockRowCap : kCtaWords;
+  constexpr size_t big_smem = sizeof(int32_t) * kWords;
   static std::atomic<uint64_t> big_attr{0};
-  if (ensure_smem_limit(k_rows_big, (int)big_smem, big_attr) != cudaSuccess) return YGX_ERR_CUDA;
-  const int64_t rows = a.rows + b.rows;
-  if (a.rows < 0 || b.rows < 0 || rows > s.stride || rows > INT32_MAX) return YGX_ERR_ARG;
-  if (cudaMemsetAsync(s.n_big, 0, 16 * sizeof(uint32_t), stream) != cudaSuccess)
+  if (ensure_smem_limit(k_rows_big<Idx>, (int)big_smem, big_attr) != cudaSuccess)
     return YGX_ERR_CUDA;
-  k_rows_classify<<<grid_for(rows, 256), 256, 0, stream>>>(a, b, s.class_rows, s.stride,
-                                                           s.n_big + 1, s.big_rows, s.n_big);
+  const int64_t rows = a.rows + b.rows;
+  k_rows_classify<<<grid_for(rows, 1024, kNumSMs * 8), 256, 0, stream>>>(a, b, s.lists, s.stride,
+                                                                         s.counts);
   YGX_CHECK_LAUNCH();
-#define YGX_ROWS(C, R)                                                                        \
-  k_rows_class<R><<<grid_small, 256, 0, stream>>>(s.class_rows + (C) * s.stride,             \
-                                                  s.n_big + 1 + (C), a, b, index_bits);       \
+  k_rows_big<Idx><<<kBigGrid, kBigThreads, big_smem, stream>>>(s.lists, s.stride, s.counts, a, b,
+                                                               s.bitmaps, universe);
   YGX_CHECK_LAUNCH();
-  YGX_ROWS(0, 1) YGX_ROWS(1, 2) YGX_ROWS(2, 4) YGX_ROWS(3, 8) YGX_ROWS(4, 16) YGX_ROWS(5, 32)
-#undef YGX_ROWS
-  k_rows_big<<<kBigGrid, kBigThreads, big_smem, stream>>>(s.big_rows, s.n_big, s.stride, a, b,
-                                                          index_bits, s.bitmaps, universe);
+  // a small tree has few rows: fewer CTAs start and end sooner
+  const int grid = grid_for(rows, 8, kNumSMs * g_tune.row_grid_per_sm);
+  k_rows_warp<Idx, 2><<<grid, 256, 0, stream>>>(a, b, s.lists, s.stride, s.counts);
+  YGX_CHECK_LAUNCH();
+  k_rows_warp<Idx, 1><<<grid, 256, 0, stream>>>(a, b, s.lists, s.stride, s.counts);
+  YGX_CHECK_LAUNCH();
+  k_rows_warp<Idx, 0><<<grid, 256, 0, stream>>>(a, b, s.lists, s.stride, s.counts);
   YGX_CHECK_LAUNCH();
   return YGX_OK;
+}
+
+int row_sort_pass(const RowSortScratch& s, const RowTable& a, const RowTable& b, int index_bits,
+                  int64_t universe, cudaStream_t stream) {
+  const int64_t rows = a.rows + b.rows;
+  if (a.rows < 0 || b.rows < 0 || rows > s.stride || rows > INT32_MAX) return YGX_ERR_ARG;
+  if (cudaMemsetAsync(s.counts, 0, 32 * sizeof(uint32_t), stream) != cudaSuccess)
+    return YGX_ERR_CUDA;
+  return index_bits == 32 ? row_sort_launch<int32_t>(s, a, b, universe, stream)
+                          : row_sort_launch<int64_t>(s, a, b, universe, stream);
 }
 
 // Entries per CTA log region for a total log capacity.
@@ -1405,7 +1273,6 @@ static TravScratch carve_trav(Arena& a, int64_t total, int64_t L, int64_t cap, i
   s.status = a.take<uint32_t>(64);
   s.stats = a.take<unsigned long long>(kStatWords);
   s.sizes = a.take<uint32_t>(kMaxGens + 2);
-  // [0] rows > kBlockRowCap, [1..6] class counts, [8] other long rows, [9] work counter
   s.n_big = a.take<uint32_t>(64);
   s.recs = a.take<NodeRec>(total);
   s.far_cnt = a.take<int32_t>(total);
@@ -1418,8 +1285,8 @@ static TravScratch carve_trav(Arena& a, int64_t total, int64_t L, int64_t cap, i
   s.far_pos = a.take<unsigned long long>(total + L);
   s.near_pos = s.far_pos ? s.far_pos + total : nullptr;
   s.scan_tmp = a.take<int64_t>(scan_scratch_elems(total > L ? total : L));
-  s.big_rows = a.take<int32_t>(total + L);  // far and near rows sort in one pass
-  s.class_rows = a.take<int32_t>((size_t)kRowClasses * (total + L));
+  // far and near rows sort in one pass
+  s.row_lists = a.take<int32_t>((size_t)kRowLists * (total + L));
   s.bitmaps = a.take<uint32_t>((size_t)kBigGrid * ((total + 31) / 32));
   s.wf[0] = a.take<int2>(region_capacity(cap) * kWalkGrid);
   s.wf[1] = a.take<int2>(region_capacity(cap) * kWalkGrid);
@@ -1913,24 +1780,24 @@ int ygx_traverse_fill_predicted(int64_t total, int64_t num_internal, int64_t wf_
     return rc;
   if ((rc = ygx::exclusive_scan<int32_t>(s.ext_near_cnt, L, s.ext_near_off, s.scan_tmp, stream)))
     return rc;
-  // moved-row lists: far rows in big_rows, near rows in class_rows (both
+  // moved-row lists: two of the row sort's lists (both
   // hold at least max(total, L) entries and are free until the finalize); counters
   // in n_big[10] / n_big[11]
   if (cudaMemsetAsync(s.n_big + 10, 0, 2 * sizeof(uint32_t), stream) != cudaSuccess)
     return YGX_ERR_CUDA;
   ygx::k_relocate_mark<<<ygx::grid_for(total, 256), 256, 0, stream>>>(
       s.pad_far, far_cap32, s.ext_far_cnt, s.ext_far_off, total, far_raw_cap, s.far_pos,
-      s.raw_off_far, s.big_rows, s.n_big + 10, s.status, ygx::kFlagFarOverflow);
+      s.raw_off_far, s.row_lists, s.n_big + 10, s.status, ygx::kFlagFarOverflow);
   YGX_CHECK_LAUNCH();
   ygx::k_relocate_mark<<<ygx::grid_for(L, 256), 256, 0, stream>>>(
       s.pad_near, near_cap32, s.ext_near_cnt, s.ext_near_off, L, near_raw_cap, s.near_pos,
-      s.raw_off_near, s.class_rows, s.n_big + 11, s.status, ygx::kFlagNearOverflow);
+      s.raw_off_near, s.row_lists + total + L, s.n_big + 11, s.status, ygx::kFlagNearOverflow);
   YGX_CHECK_LAUNCH();
-  ygx::k_relocate_copy<<<ygx::kNumSMs * 8, 256, 0, stream>>>(s.big_rows, s.n_big + 10, s.pad_far,
+  ygx::k_relocate_copy<<<ygx::kNumSMs * 8, 256, 0, stream>>>(s.row_lists, s.n_big + 10, s.pad_far,
                                                             far_cap32, s.raw_off_far, far_raw32);
   YGX_CHECK_LAUNCH();
   ygx::k_relocate_copy<<<ygx::kNumSMs * 8, 256, 0, stream>>>(
-      s.class_rows, s.n_big + 11, s.pad_near, near_cap32, s.raw_off_near, near_raw32);
+      s.row_lists + total + L, s.n_big + 11, s.pad_near, near_cap32, s.raw_off_near, near_raw32);
   YGX_CHECK_LAUNCH();
   ygx::k_raw_ends<<<ygx::grid_for(total, 256), 256, 0, stream>>>(s.raw_off_far, s.far_cnt, total,
                                                                  s.raw_end_far);
@@ -1997,7 +1864,7 @@ static int finalize_impl(const ygx::TravScratch& s, int64_t total, int64_t L,
                          const int32_t* near_row_base, void* far_sources, void* far_targets,
                          void* target_levels, void* neighbors, void* neighbor_leaf_positions,
                          int64_t max_nbr, cudaStream_t stream) {
-  const ygx::RowSortScratch rs{s.n_big, s.big_rows, s.class_rows, s.bitmaps, total + L};
+  const ygx::RowSortScratch rs{s.n_big, s.row_lists, s.bitmaps, total + L};
   const ygx::RowTable far_rows{total, s.far_off, s.far_cnt, level32, far_src32, far_raw_off,
                                far_row_base, far_sources, far_targets, target_levels};
   const ygx::RowTable near_rows{L, s.near_off, s.near_cnt, nullptr, near_nbr32, near_raw_off,
