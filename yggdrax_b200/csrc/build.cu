@@ -106,6 +106,40 @@ __global__ void __launch_bounds__(kReorderThreads)
   }
 }
 
+// inverse[order[k]] = k for a table larger than the L2 keeps: its writes hit
+// random sectors, and a sector that leaves the L2 with one entry written is
+// read back from DRAM for the next.  So the table is written window by window
+// (CTAs start in the order of their index), reading the whole order for each.
+// Small windows stay in the L2, but each costs a read of the order: 16 MB up
+// to 8 of them, then larger ones up to 64 MB.  The whole reorder (packed
+// particles, 64-bit indices, random order), us:
+//   n            one pass   windows of 16 MB   32 MB   64 MB
+//    1,048,576        18          (one window: one pass)
+//    4,194,304       102                 91     102     102
+//    6,291,456       232                154     171     231
+//   16,777,216       917                512     565     578
+//   33,554,432      2094               1414    1314    1293
+constexpr int64_t kInverseWindow = 16 << 20, kInverseWindowMax = 64 << 20;  // bytes
+constexpr int64_t kInverseWindows = 8;
+__global__ void __launch_bounds__(kReorderThreads)
+    k_inverse_windows(const uint32_t* __restrict__ order, int64_t n, int64_t window, int64_t chunks,
+                      int index_bits, void* __restrict__ inverse) {
+  const int64_t lo = (int64_t)blockIdx.x / chunks * window;
+  const int64_t k0 = (int64_t)blockIdx.x % chunks * (kReorderThreads * kReorderItems) + threadIdx.x;
+  uint32_t v[kReorderItems];
+#pragma unroll
+  for (int u = 0; u < kReorderItems; ++u) {
+    const int64_t k = k0 + (int64_t)u * kReorderThreads;
+    v[u] = k < n ? order[k] : 0u;
+  }
+#pragma unroll
+  for (int u = 0; u < kReorderItems; ++u) {
+    const int64_t k = k0 + (int64_t)u * kReorderThreads;
+    if (k < n && (int64_t)v[u] >= lo && (int64_t)v[u] < lo + window)
+      store_idx(inverse, index_bits, v[u], k);
+  }
+}
+
 // _tree_impl.py:405-406: fixed-size chunks of the sorted order.
 __global__ void k_leaves_adaptive(const uint64_t* __restrict__ codes, int64_t n, int64_t leaf_size,
                                   int64_t L, int index_bits, void* starts, void* ends,
@@ -897,32 +931,57 @@ int ygx_pack_particles(const float* positions, const float* masses, int64_t n, v
   return YGX_OK;
 }
 
+// The inverse if it is to be written after the reorder, in windows; null if
+// the reorder writes it itself (one window holds it, or none is wanted).
+static void* inverse_after(int64_t n, int index_bits, void* inverse) {
+  return n * (index_bits / 8) > ygx::kInverseWindow ? inverse : nullptr;
+}
+static int write_inverse(const uint32_t* order, int64_t n, int index_bits, void* inverse,
+                         cudaStream_t stream) {
+  constexpr int64_t kChunk = (int64_t)ygx::kReorderThreads * ygx::kReorderItems;
+  const int64_t bytes = n * (index_bits / 8);
+  int64_t windows = (bytes + ygx::kInverseWindow - 1) / ygx::kInverseWindow;
+  if (windows > ygx::kInverseWindows) {
+    windows = (bytes + ygx::kInverseWindowMax - 1) / ygx::kInverseWindowMax;
+    if (windows < ygx::kInverseWindows) windows = ygx::kInverseWindows;
+  }
+  const int64_t window = (n + windows - 1) / windows;
+  const int64_t chunks = (n + kChunk - 1) / kChunk;
+  if (windows * chunks > INT32_MAX) return YGX_ERR_ARG;
+  ygx::k_inverse_windows<<<(unsigned)(windows * chunks), ygx::kReorderThreads, 0, stream>>>(
+      order, n, window, chunks, index_bits, inverse);
+  YGX_CHECK_LAUNCH();
+  return YGX_OK;
+}
+
 int ygx_reorder_packed(const void* packed, const uint32_t* order, int64_t n, int index_bits,
                        float* positions_sorted, float* masses_sorted, void* particle_indices,
                        void* inverse, cudaStream_t stream) {
   if (n < 1 || !order || !packed || (reinterpret_cast<uintptr_t>(packed) & 15u) != 0 ||
       (index_bits != 32 && index_bits != 64))
     return YGX_ERR_ARG;
+  void* late = inverse_after(n, index_bits, inverse);
   ygx::k_reorder_packed<<<ygx::grid_for((n + ygx::kReorderItems - 1) / ygx::kReorderItems,
                                          ygx::kReorderThreads),
                           ygx::kReorderThreads, 0, stream>>>(
       reinterpret_cast<const float4*>(packed), order, n, index_bits, positions_sorted,
-      masses_sorted, particle_indices, inverse);
+      masses_sorted, particle_indices, late ? nullptr : inverse);
   YGX_CHECK_LAUNCH();
-  return YGX_OK;
+  return late ? write_inverse(order, n, index_bits, late, stream) : YGX_OK;
 }
 
 int ygx_reorder(const float* positions, const float* masses, const uint32_t* order, int64_t n,
                 int index_bits, float* positions_sorted, float* masses_sorted,
                 void* particle_indices, void* inverse, cudaStream_t stream) {
   if (n < 1 || !order || (index_bits != 32 && index_bits != 64)) return YGX_ERR_ARG;
+  void* late = inverse_after(n, index_bits, inverse);
   ygx::k_reorder<<<ygx::grid_for((n + ygx::kReorderItems - 1) / ygx::kReorderItems,
                                   ygx::kReorderThreads),
                    ygx::kReorderThreads, 0, stream>>>(
       positions, masses, order, n, index_bits, positions_sorted, masses_sorted, particle_indices,
-      inverse);
+      late ? nullptr : inverse);
   YGX_CHECK_LAUNCH();
-  return YGX_OK;
+  return late ? write_inverse(order, n, index_bits, late, stream) : YGX_OK;
 }
 
 int ygx_leaves_adaptive(const uint64_t* codes_sorted, int64_t n, int64_t leaf_size, int index_bits,
