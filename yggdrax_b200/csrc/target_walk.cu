@@ -1306,19 +1306,34 @@ struct TwPad {
 
 // Dense neighbour leaf positions (L x max_nbr, -1 padded) of
 // _result_to_neighbors (:3658-3688).
-// One warp per row: no division, whole sectors written.  263,480 rows of 98
-// (the 4,194,304-particle fixed-depth octree): 130 -> 94 us.
+// A warp per 128 columns of a row, four entries in flight per lane: bound by
+// the table's writes when it is large, by the two gathers per entry otherwise.
+// Against a warp per row, one entry in flight: 263,480 rows of 98 (fixed-depth
+// octree of 4,194,304 particles) 94 -> 73 us (98 with eight in flight), 4,096
+// rows of 65,536 particles 100 -> 27, 500 rows 10.5 -> 2.2.
+template <typename Idx>
 __global__ void k_tw_nbr_leaf_pos(const int64_t* __restrict__ near_off,
                                   const int32_t* __restrict__ near_cnt, int64_t L,
-                                  const void* neighbors, int index_bits,
-                                  const int32_t* __restrict__ leafpos, int64_t max_nbr, void* out) {
+                                  const Idx* __restrict__ neighbors,
+                                  const int32_t* __restrict__ leafpos, int64_t max_nbr,
+                                  Idx* __restrict__ out) {
+  constexpr int kU = 4;
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < L; j += nw) {
-    const int64_t off = near_off[j], cnt = near_cnt[j], o = j * max_nbr;
-    for (int64_t k = lane; k < max_nbr; k += 32)
-      store_idx(out, index_bits, o + k,
-                k < cnt ? leafpos[load_idx(neighbors, index_bits, off + k)] : -1);
+  const int64_t parts = (max_nbr + 32 * kU - 1) / (32 * kU);
+  for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < L * parts; w += nw) {
+    const int64_t j = parts == 1 ? w : w / parts, k0 = (w - j * parts) * (32 * kU) + lane;
+    const int64_t off = near_off[j], cnt = near_cnt[j];
+    Idx v[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+      v[u] = k0 + u * 32 < cnt ? neighbors[off + k0 + u * 32] : (Idx)-1;
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+      if (v[u] >= 0) v[u] = (Idx)leafpos[v[u]];
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+      if (k0 + u * 32 < max_nbr) out[j * max_nbr + k0 + u * 32] = v[u];
   }
 }
 
@@ -1963,9 +1978,15 @@ static int walk_lists(bool forest, const int32_t* far_row_base, const int32_t* n
     }
   }
   if (max_nbr > 0 && neighbor_leaf_positions && leafpos32 && L > 0) {
-    k_tw_nbr_leaf_pos<<<grid_for(L * 32, 256), 256, 0, stream>>>(
-        s.near_off, s.near_cnt, L, neighbors, index_bits, leafpos32, max_nbr,
-        neighbor_leaf_positions);
+    const int grid = grid_for(L * ((max_nbr + 127) / 128) * 32, 256, kNumSMs * 64);
+    if (index_bits == 32)
+      k_tw_nbr_leaf_pos<<<grid, 256, 0, stream>>>(
+          s.near_off, s.near_cnt, L, (const int32_t*)neighbors, leafpos32, max_nbr,
+          (int32_t*)neighbor_leaf_positions);
+    else
+      k_tw_nbr_leaf_pos<<<grid, 256, 0, stream>>>(
+          s.near_off, s.near_cnt, L, (const int64_t*)neighbors, leafpos32, max_nbr,
+          (int64_t*)neighbor_leaf_positions);
     YGX_CHECK_LAUNCH();
   }
   return YGX_OK;
