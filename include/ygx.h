@@ -60,8 +60,10 @@ enum {
 #define YGX_TUNE_SPIN_LIMIT 6  /* iterations a device-side wait (sort look-back) spins   */
                                /* before it gives up and flags YGX_FLAG_TIMEOUT          */
                                /* (0..2^24; default 2^22); not a performance knob        */
-#define YGX_TUNE_TARGET_BUDGET 7 /* steps one warp spends on a piece of a target before */
-                                 /* handing the rest to other warps (1..4096; 128)     */
+#define YGX_TUNE_TARGET_BUDGET 7 /* steps (64 candidates each; 32 in the ordered walk and */
+                                 /* past 2^24 nodes) one warp spends on a piece of a     */
+                                 /* target before handing the rest to other warps        */
+                                 /* (1..4096; 128)                                       */
 #define YGX_TUNE_SORT_BITS 8   /* onesweep digit width: 8, or 11 (2048 bins) for every  */
                                /* sort whose key range it covers in fewer passes        */
                                /* (63-bit Morton codes: 6 passes instead of 8)          */

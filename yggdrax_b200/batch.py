@@ -426,7 +426,10 @@ def _target_lists_batched(batch: BatchedTrees, geometry: BatchedGeometry, theta:
         if f & (L.FLAG_TIMEOUT | L.FLAG_MALFORMED):
             return None
         if f & L.FLAG_LOG_OVERFLOW:
-            caps = _grow_target_caps(caps, needs, runs, f)
+            try:
+                caps = _grow_target_caps(caps, needs, runs, f)
+            except L.YgxError:
+                return None
             ws = None
             continue
         if f:

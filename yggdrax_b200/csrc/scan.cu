@@ -113,6 +113,5 @@ int exclusive_scan(const InT* in, int64_t n, int64_t* out, int64_t* tmp, cudaStr
 
 template int exclusive_scan<int32_t>(const int32_t*, int64_t, int64_t*, int64_t*, cudaStream_t);
 template int exclusive_scan<int64_t>(const int64_t*, int64_t, int64_t*, int64_t*, cudaStream_t);
-template int exclusive_scan<uint32_t>(const uint32_t*, int64_t, int64_t*, int64_t*, cudaStream_t);
 
 }  // namespace ygx

@@ -786,7 +786,6 @@ __global__ void k_near_offsets(const int64_t* __restrict__ off, const int32_t* _
 constexpr int kBlockRowCap = 16384; // one CTA, 64 KB of shared memory
 constexpr int kBigThreads = kCtaThreads;
 
-template <bool kBlockSync>
 __device__ __forceinline__ void mirrored_bitonic(int32_t* a, int64_t n64, int tid, int nthreads) {
   // Row lengths stay below 2^31 (they are counts of one node's partners).
   const int32_t n = (int32_t)n64;
@@ -806,7 +805,7 @@ __device__ __forceinline__ void mirrored_bitonic(int32_t* a, int64_t n64, int ti
           if (x > y) { a[lo] = y; a[hi] = x; }
         }
       }
-      if (kBlockSync) __syncthreads(); else __syncwarp();
+      __syncthreads();
     }
   }
 }
@@ -1137,13 +1136,13 @@ __global__ void __launch_bounds__(kBigThreads, 1)
         int32_t* a = reinterpret_cast<int32_t*>(s_dyn);
         for (int64_t k = tid; k < n; k += nt) a[k] = raw[roff + k];
         __syncthreads();
-        mirrored_bitonic<true>(a, n, tid, nt);
+        mirrored_bitonic(a, n, tid, nt);
         emit_row(a, n, off, index_bits, vals_out, tgt_out, lvl_out, r - vbase, vbase, lvl, tid, nt);
         __syncthreads();
         for (int64_t k = tid; k < n; k += nt) s_dyn[k] = 0u;  // bitmap stays zero
       } else {
         int32_t* a = raw + roff;
-        mirrored_bitonic<true>(a, n, tid, nt);
+        mirrored_bitonic(a, n, tid, nt);
         emit_row(a, n, off, index_bits, vals_out, tgt_out, lvl_out, r - vbase, vbase, lvl, tid, nt);
       }
     }
