@@ -468,9 +468,12 @@ __device__ __noinline__ void pw_join_split(const PwArgs& a, PwWarpSmem& W, int t
 // Warp-collective: the stack and the source candidates from `cur` on become
 // continuation pieces for other warps.  A target that was run by one warp so
 // far becomes shared first: its counts go to the row counters and its split
-// list becomes the first chunk.
+// list becomes the first chunk.  The row's place may still be on its way here: a
+// leaf target can be handed off before anything was flushed (budget 1, a stack
+// full after a few refining windows, hungry warps), so the copy is waited for.
 __device__ __noinline__ void pw_hand_off(const PwArgs& a, PwWarpSmem& W, const PwPiece pc, int t,
                                          int t_leaf, int cur, int stk_n, int lane) {
+  pw_copy_wait();  // (lane 0 issued the copy and reads the row)
   const int shared = (pc.flags & kPwShared) != 0;
   if (!shared) {
     const int s_len = t_leaf ? 0 : W.s_len;
@@ -691,7 +694,7 @@ __device__ __forceinline__ bool pw_run_piece(const PwArgs& a, PwSmem& sm, PwWarp
       break;
     }
   }
-  pw_copy_wait();  // also where nothing is flushed: the next piece reuses the rows
+  pw_copy_wait();  // also where nothing is flushed: the row is read and reused after this
   tot_a += n_a;
   tot_b += n_b;
   pw_flush_row(a, W, 0, shared, n_a, lane);
