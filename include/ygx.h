@@ -209,7 +209,8 @@ size_t ygx_topology_workspace_size(int64_t num_leaves);
  * nodes_by_level, num_levels (1) -- plus int32 copies used by the geometry
  * and traversal kernels (left32/right32 span all nodes, -1 on leaves).
  * *tree_flags_out (device word) gets YGX_FLAG_MALFORMED when tied leaf codes
- * produced a parent array that disagrees with the child arrays. */
+ * produced a parent array that disagrees with the child arrays, and
+ * YGX_FLAG_TIMEOUT when a wait gave up (the tables are then incomplete). */
 int ygx_build_topology(const uint64_t* leaf_codes, const void* leaf_starts, const void* leaf_ends,
                        int64_t L, int index_bits, void* parent, void* left, void* right,
                        uint8_t* left_is_leaf, uint8_t* right_is_leaf, void* node_ranges,

@@ -461,8 +461,9 @@ struct TopoArgs {
   uint32_t* hist;        // per bin, per CTA
   int32_t* by_low;       // nodes by the low digit of their level (two-digit levels)
   int32_t* max_level;    // zeroed
-  uint32_t* tree_flags;  // zeroed
-  uint32_t* tree_flags_out;
+  // zeroed, ORed into by any CTA and never stored to: a CTA that gives up at the
+  // last barrier reports it there while others, which passed it, finish
+  uint32_t* tree_flags;
   uint32_t* status;
   DepthArgs depth;
 };
@@ -635,7 +636,6 @@ __device__ bool build_topology(const TopoArgs& a) {
     }
     const int64_t nl = (int64_t)deepest + 1;
     store_idx(a.num_levels, ib, 0, nl < 1 ? 1 : (nl > 64 ? 64 : nl));
-    if (a.tree_flags_out) *a.tree_flags_out = __ldcg(a.tree_flags);
   }
   return true;
 }
@@ -643,7 +643,7 @@ __device__ bool build_topology(const TopoArgs& a) {
 __global__ void __launch_bounds__(kGenThreads, 2) k_topology(const TopoArgs a) {
   if (!build_topology(a) && threadIdx.x == 0) {
     raise_flag(a.status, kFlagTimeout);
-    if (a.tree_flags_out) atomicExch(a.tree_flags_out, kFlagTimeout);
+    raise_flag(a.tree_flags, kFlagTimeout);
   }
 }
 
@@ -1077,7 +1077,8 @@ size_t ygx_topology_workspace_size(int64_t num_leaves) {
 // (total), num_levels (1); bool flags (L-1); int32 traversal copies
 // parent32/left32/right32/level32 (total, -1 children for leaves) and
 // nbl32 (total).  tree_flags_out (device, 1 word) receives kFlagMalformed
-// when the parent array and the child arrays disagree.
+// when the parent array and the child arrays disagree, kFlagTimeout when a wait
+// gave up.
 int ygx_build_topology(const uint64_t* leaf_codes, const void* leaf_starts, const void* leaf_ends,
                        int64_t L, int index_bits, void* parent, void* left, void* right,
                        uint8_t* left_is_leaf, uint8_t* right_is_leaf, void* node_ranges,
@@ -1091,8 +1092,8 @@ int ygx_build_topology(const uint64_t* leaf_codes, const void* leaf_starts, cons
   ygx::Arena a{(char*)ws, 0, ws_bytes};
   ygx::TopoScratch s = ygx::carve_topo(a, L);
   const int64_t total = 2 * L - 1;
-  // flags, barrier and maximum are contiguous: one memset
-  if (cudaMemsetAsync(s.tree_flags, 0, (char*)(s.max_level + 64) - (char*)s.tree_flags, stream) !=
+  // status, flags, barrier and maximum are contiguous: one memset
+  if (cudaMemsetAsync(s.status, 0, (char*)(s.max_level + 64) - (char*)s.status, stream) !=
       cudaSuccess)
     return YGX_ERR_CUDA;
   int bl = 0;  // the reference's doubling rounds: bit_length(total) + 1
@@ -1123,12 +1124,17 @@ int ygx_build_topology(const uint64_t* leaf_codes, const void* leaf_starts, cons
   t.by_low = s.parent_claim;  // free once the parents are known
   t.max_level = s.max_level;
   t.tree_flags = s.tree_flags;
-  t.tree_flags_out = tree_flags_out;
   t.status = s.status;
   t.depth = ygx::DepthArgs{parent32, total,  bl + 1,    level32,
                            s.sc[0],  s.sc[1], s.d[1],   s.deep,
                            s.arrived, (uint32_t)ygx::g_tune.spin_limit};
-  return ygx::launch_cooperative(ygx::k_topology, t, total, stream);
+  const int rc = ygx::launch_cooperative(ygx::k_topology, t, total, stream);
+  if (rc) return rc;
+  if (tree_flags_out &&
+      cudaMemcpyAsync(tree_flags_out, s.tree_flags, sizeof(uint32_t), cudaMemcpyDeviceToDevice,
+                      stream) != cudaSuccess)
+    return YGX_ERR_CUDA;
+  return YGX_OK;
 }
 
 
