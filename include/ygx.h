@@ -586,7 +586,8 @@ size_t ygx_batch_topology_workspace_size(int64_t total_leaves, int64_t S);
  * nodes_by_level: 2 total_leaves - S; left / right / flags: total_leaves - S;
  * level_offsets S x 65; num_levels S), int32 copies with global node ids,
  * node_seg32 / leafpos32 / node_base32 (per node), leaf_base32 (per leaf),
- * seg_flags (S) and their union tree_flags_out. */
+ * seg_flags (S: YGX_FLAG_MALFORMED per set; YGX_FLAG_TIMEOUT in all of them
+ * when a wait gave up) and their union tree_flags_out. */
 int ygx_batch_build_topology(const uint64_t* leaf_codes, const void* leaf_starts,
                              const void* leaf_ends, const int64_t* leaf_off,
                              const int32_t* leaf_seg, int64_t S, int64_t total_leaves,

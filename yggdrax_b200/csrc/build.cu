@@ -835,10 +835,15 @@ __global__ void k_seg_depth_finish(const int32_t* __restrict__ sc, const int32_t
   }
 }
 
+// Level tables of every set.  Depths whose barrier gave up are no set's: the
+// timeout goes to every set's flags, which the walks over the forest read.
 __global__ void k_seg_level_tables(const uint32_t* __restrict__ seg_hist,
                                    const int32_t* __restrict__ seg_max,
                                    const int64_t* __restrict__ leaf_off, int64_t S,
-                                   int index_bits, void* level_offsets, void* num_levels) {
+                                   int index_bits, void* level_offsets, void* num_levels,
+                                   const uint32_t* __restrict__ tree_flags,
+                                   uint32_t* __restrict__ seg_flags) {
+  const uint32_t timeout = *tree_flags & kFlagTimeout;
   for (int64_t sg = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; sg < S;
        sg += (int64_t)gridDim.x * blockDim.x) {
     // a one-leaf tree has the reference's literal table (_tree_impl.py:1052-1110)
@@ -852,6 +857,7 @@ __global__ void k_seg_level_tables(const uint32_t* __restrict__ seg_hist,
     int64_t nl = (int64_t)seg_max[sg] + 1;
     nl = nl < 1 ? 1 : (nl > 64 ? 64 : nl);
     store_idx(num_levels, index_bits, sg, nl);
+    if (timeout) atomicOr(&seg_flags[sg], timeout);
   }
 }
 
@@ -1246,7 +1252,8 @@ size_t ygx_batch_topology_workspace_size(int64_t total_leaves, int64_t S) {
 // set of every node, leafpos32 the near-row position of every leaf (the
 // sets' leaves back to back; -1 for internal nodes), node_base32 / leaf_base32
 // the first node id of the set of every node / leaf, seg_flags (S)
-// YGX_FLAG_MALFORMED per set and tree_flags_out (1 word) their union.
+// YGX_FLAG_MALFORMED per set (and YGX_FLAG_TIMEOUT in all, when a wait gave up)
+// and tree_flags_out (1 word) their union.
 int ygx_batch_build_topology(const uint64_t* leaf_codes, const void* leaf_starts,
                              const void* leaf_ends, const int64_t* leaf_off,
                              const int32_t* leaf_seg, int64_t S, int64_t total_leaves,
@@ -1293,7 +1300,8 @@ int ygx_batch_build_topology(const uint64_t* leaf_codes, const void* leaf_starts
       s.seg_hist, s.seg_max, seg_flags, s.tree_flags);
   YGX_CHECK_LAUNCH();
   ygx::k_seg_level_tables<<<ygx::grid_for(S, 128), 128, 0, stream>>>(
-      s.seg_hist, s.seg_max, leaf_off, S, index_bits, level_offsets, num_levels);
+      s.seg_hist, s.seg_max, leaf_off, S, index_bits, level_offsets, num_levels, s.tree_flags,
+      seg_flags);
   YGX_CHECK_LAUNCH();
   // nodes_by_level: stable sort by (set, level); sets < 2^16, levels < 2^16
   rc = ygx::onesweep_sort(s.level_keys, nullptr, total, 0, 32, s.level_keys_sorted, s.nbl_u32,

@@ -275,8 +275,9 @@ __global__ void k_pw_forest_slots(const float* __restrict__ center,
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < S;
        q += (int64_t)gridDim.x * blockDim.x) {
     if (leaf_off[q + 1] - leaf_off[q] < 2) continue;
-    if (seg_flags[q] & kFlagMalformed) {  // no tree to walk: nothing of it is queued
-      raise_flag(status, kFlagMalformed);
+    // no tree to walk, or one whose build gave up: nothing of it is queued
+    if (const uint32_t f = seg_flags[q] & (kFlagMalformed | kFlagTimeout)) {
+      raise_flag(status, f);
       ctl->stop = 1u;
       ctl->q_head = q_cap;  // no warp takes a piece of any set
       continue;

@@ -646,6 +646,7 @@ __global__ void k_seed_forest(int2* wf, uint32_t* cnt, uint32_t* sizes, uint32_t
   for (int64_t sg = threadIdx.x; sg < S; sg += blockDim.x) {
     const int64_t a = leaf_off[sg], Ls = leaf_off[sg + 1] - a, NO = 2 * a - sg;
     int64_t root = NO;
+    if (seg_flags && (seg_flags[sg] & kFlagTimeout)) raise_flag(status, kFlagTimeout);
     if (seg_flags && (seg_flags[sg] & kFlagMalformed)) {
       for (int64_t k = NO; k < NO + 2 * Ls - 1; ++k)
         if (parent32[k] < 0) { root = k; break; }
