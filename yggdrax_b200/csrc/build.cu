@@ -1238,8 +1238,8 @@ static SegTopoScratch carve_seg_topo(ygx::Arena& a, int64_t total, int64_t S) {
 
 size_t ygx_batch_topology_workspace_size(int64_t total_leaves, int64_t S) {
   ygx::Arena a{nullptr, 0, 0};
-  const int64_t total = total_leaves > S ? 2 * total_leaves - S : 1;
-  carve_seg_topo(a, total, S > 0 ? S : 1);
+  const int64_t total = 2 * total_leaves - S;  // (as many as sets when each is one leaf)
+  carve_seg_topo(a, total > 0 ? total : 1, S > 0 ? S : 1);
   return a.used + 256;
 }
 
