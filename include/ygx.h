@@ -752,14 +752,15 @@ int ygx_octree_view(const uint8_t* valid, const uint8_t* leaf, const uint64_t* c
  * -1.  mac 0 bh (box max extent), 1 dehnen (box radius x scale), 2 engblom
  * (box radius).  Every accepted (near) pair is logged twice, per generation
  * first as (row of t, s) then as (row of s, t), into *_key / *_val
- * (log_capacity entries); *_cnt receive the row lengths.  stats_out (host,
- * 8 x int64): far log entries, near log entries, accept, near, refine
- * decisions, generations, the largest wavefront kept.  flags_out (host):
- * bit 0 a far row above far_row_cap, bit 1 a near row above near_row_cap,
- * bit 2 more children than max_pair_queue (the walk stops after that
- * generation, like the reference), bit 4 more children than wf_capacity
- * (re-run with stats_out[6] or more), bit 5 the log was too short (the walk
- * ran on; re-run with stats_out[0] or [1] entries).  Synchronizes once per
+ * (log_capacity entries); far_cnt (M) receives the row length of every cell
+ * by cell, near_cnt (near_rows) by row.  stats_out (host, 8 x int64): far log
+ * entries, near log entries, accept, near, refine decisions, generations, the
+ * largest wavefront kept.  flags_out (host): bit 0 a far row above
+ * far_row_cap, bit 1 a near row above near_row_cap, bit 2 more children than
+ * max_pair_queue (the walk stops after that generation, like the reference),
+ * bit 4 more children than wf_capacity (re-run with stats_out[6] or more),
+ * bit 5 the log was too short (the walk ran on; re-run with stats_out[0] or
+ * [1] entries).  Synchronizes once per
  * generation.  A stable sort of the log by key gives the reference's rows. */
 size_t ygx_octree_walk_workspace_size(int64_t M, int64_t wf_capacity);
 int ygx_octree_walk(const void* children, const void* child_counts, int index_bits, int64_t M,

@@ -151,11 +151,12 @@ __device__ __forceinline__ int oct_child_count(const OctArgs& p, uint8_t kind, i
 }
 
 // Writes one accepted / near pair to both blocks of its log and counts both
-// rows.  A row past its capacity and a log that is too short are flagged.
+// rows, at counter n.x and n.y.  A row past its capacity and a log that is too
+// short are flagged.
 __device__ __forceinline__ unsigned oct_log(uint64_t* key, uint32_t* val, int64_t log_cap,
                                             long long fwd, long long bwd, int32_t row_t,
-                                            int32_t row_s, int2 w, int32_t* cnt, int64_t cap,
-                                            unsigned over) {
+                                            int32_t row_s, int2 w, int32_t* cnt, int2 n,
+                                            int64_t cap, unsigned over) {
   unsigned f = 0;
   if (bwd < log_cap) {
     key[fwd] = (uint64_t)(uint32_t)row_t;
@@ -165,8 +166,8 @@ __device__ __forceinline__ unsigned oct_log(uint64_t* key, uint32_t* val, int64_
   } else {
     f |= kOctLogShort;
   }
-  if ((int64_t)atomicAdd(&cnt[row_t], 1) >= cap) f |= over;
-  if ((int64_t)atomicAdd(&cnt[row_s], 1) >= cap) f |= over;
+  if ((int64_t)atomicAdd(&cnt[n.x], 1) >= cap) f |= over;
+  if ((int64_t)atomicAdd(&cnt[n.y], 1) >= cap) f |= over;
   return f;
 }
 
@@ -230,16 +231,17 @@ __global__ void __launch_bounds__(kGenThreads, 2) k_oct_walk(const OctArgs a) {
       unsigned long long sum;
       const unsigned long long at = gen_block_scan(v, &sum);
       if (kd == kOctFar) {
+        // counted by cell: a cell's row key is the caller's and only sorted by
         const long long r = far_n + (long long)pre.x + (long long)((at >> 32) & 0xffffull);
         raise |= oct_log(a.far_key, a.far_val, a.log_cap, r, r + (long long)all.x,
-                         a.far_row[w.x], a.far_row[w.y], w, a.far_cnt, a.far_cap, kOctFarOver);
+                         a.far_row[w.x], a.far_row[w.y], w, a.far_cnt, w, a.far_cap, kOctFarOver);
       } else if (kd == kOctNear) {
         const long long r = near_n + (long long)pre.y + (long long)(at >> 48);
         const int32_t rt = a.near_row[w.x], rs = a.near_row[w.y];
         if (rt < 0 || rs < 0) raise |= kOctBadInput;
         else
           raise |= oct_log(a.near_key, a.near_val, a.log_cap, r, r + (long long)all.y, rt, rs, w,
-                           a.near_cnt, a.near_cap, kOctNearOver);
+                           a.near_cnt, make_int2(rt, rs), a.near_cap, kOctNearOver);
       } else if (kd) {
         int64_t slot = (int64_t)pre.child + (int64_t)(at & 0xffffffffull);
         auto put = [&](int x, int y) {
