@@ -730,6 +730,7 @@ __global__ void __launch_bounds__(kPwThreads, kPwBlocksPerSM)
   const unsigned lt = lanemask_lt_();
   unsigned fin = 0;   // targets this warp finished and has not reported (lane 0)
   bool have = false;  // pc holds the next piece (a finished target's left child)
+  int room = 1;       // whether its sibling was queued (lane 0)
   PwPiece pc;
   while (true) {
     if (!have) {
@@ -818,9 +819,16 @@ __global__ void __launch_bounds__(kPwThreads, kPwBlocksPerSM)
       W.st.busy += (unsigned long long)(now - W.t_mark);
       W.t_mark = now;
     }
-    if (complete && !t_leaf) {
-      // both children inherit the split list: the right one is queued, this
-      // warp goes on with the left one
+    // both children inherit the split list: the right one is queued, this warp
+    // goes on with the left one.  Not after a push that found no room: the walk
+    // is re-run with a longer queue anyway, and a chain of left children that no
+    // queue entry pays for ends only if the tree does (the children that a C
+    // caller gives may form a cycle).  The push before is the one looked at,
+    // so that nothing waits for this one's round trip (walk of 16 M particles
+    // 7.23 -> 7.25 ms, of 1 M 0.77 -> 0.78).
+    const bool go = complete && !t_leaf && __shfl_sync(0xffffffffu, room, 0) != 0;
+    room = 1;
+    if (go) {
       pc.et = (2u * (uint32_t)t) | ((pc.et & ~kPwSlotMask) + kPwGen);
       pc.flags = kPwSibling;
       pc.n_spill = 0;
@@ -836,6 +844,7 @@ __global__ void __launch_bounds__(kPwThreads, kPwBlocksPerSM)
           a.queue[qs] = q;
           pw_store_release(&a.q_ready[qs], 1u);
         } else {
+          room = 0;
           raise_flag(a.status, kFlagLogOverflow);
           a.ctl->stop = 1u;
         }
