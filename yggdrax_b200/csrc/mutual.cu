@@ -71,7 +71,7 @@ __global__ void k_mut_prepare(const void* __restrict__ left, const void* __restr
 __device__ __forceinline__ uint8_t mut_evaluate(const MutualArgs& a, int2 p, bool* bad) {
   const int32_t sa = p.x, sb = p.y;
   if (!(sa >= 0 && sb >= 0 && sa < a.total && sb < a.total)) {
-    *bad = sa >= a.total || sb >= a.total;
+    *bad |= sa >= a.total || sb >= a.total;
     return 0;
   }
   const float4 A = a.rec[sa], B = a.rec[sb];
