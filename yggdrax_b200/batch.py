@@ -385,7 +385,7 @@ def build_interactions_and_neighbors_batched(batch: BatchedTrees, geometry: Batc
 
 # First capacities of a forest's per-target walk, entries per node (far, near
 # and split entries, continuations, records of the three, queue): sets of up
-# to some 20,000 particles fit, and 8 M nodes take 14 GB; what a walk needed
+# to some 20,000 particles fit, and 8 M nodes take 22 GB; what a walk needed
 # then sizes the next one.
 _BATCH_FIRST_CAPS = [84.0, 140.0, 140.0, 14.0, 6.0, 6.0, 6.0, 4.0]
 

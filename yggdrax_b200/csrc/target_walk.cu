@@ -1451,17 +1451,20 @@ static TwScratch carve_tw(Arena& a, int64_t total, int64_t L, const TwCaps& c, b
   s.near_keys = a.take<unsigned long long>(c.near_rec);
   s.near_recs = a.take<TwChunk>(c.near_rec);
   s.s_recs = a.take<TwSChunk>(c.s_rec);
-  const int64_t mrec = c.far_rec > c.near_rec ? c.far_rec : c.near_rec;
-  s.order = a.take<uint32_t>(mrec);
-  s.keys_sorted = a.take<unsigned long long>(mrec);
-  s.sorted_cnt = a.take<int32_t>(mrec);
-  s.dest = a.take<int64_t>(mrec + 1);
-  const size_t plan = seg_scan_elems(total, 4);
-  const size_t chunks = scan_scratch_elems(mrec);
-  s.scan_tmp = a.take<int64_t>(plan > chunks ? plan : chunks);
+  size_t scan = seg_scan_elems(total, 4);
+  if (ordered) {  // the chunks' records are sorted
+    const int64_t mrec = c.far_rec > c.near_rec ? c.far_rec : c.near_rec;
+    s.order = a.take<uint32_t>(mrec);
+    s.keys_sorted = a.take<unsigned long long>(mrec);
+    s.sorted_cnt = a.take<int32_t>(mrec);
+    s.dest = a.take<int64_t>(mrec + 1);
+    const size_t chunks = scan_scratch_elems(mrec);
+    scan = scan > chunks ? scan : chunks;
+    s.sort_ws_bytes = onesweep_scratch_bytes(mrec) + 256;
+    s.sort_ws = a.take<unsigned char>(s.sort_ws_bytes);
+  }
+  s.scan_tmp = a.take<int64_t>(scan);
   s.near_off = a.take<int64_t>((L > 0 ? L : 1) + 1);
-  s.sort_ws_bytes = onesweep_scratch_bytes(mrec) + 256;
-  s.sort_ws = a.take<unsigned char>(s.sort_ws_bytes);
   s.far_off_node = nullptr;
   s.first_ovf_far = s.first_ovf_near = nullptr;
   s.ext_far = s.ext_near = s.roff_far = s.roff_near = nullptr;
