@@ -377,7 +377,10 @@ def build_interactions_and_neighbors_batched(batch: BatchedTrees, geometry: Batc
         raise ValueError("dehnen_radius_scale must be > 0")
     total = batch.total_nodes
     if total >= 3 and batch.total_leaves > batch.num_sets and 2 * total <= _PAIR_WALK_MAX_NODES:
-        out = _target_lists_batched(batch, geometry, theta, mac_type, dehnen_radius_scale)
+        try:
+            out = _target_lists_batched(batch, geometry, theta, mac_type, dehnen_radius_scale)
+        except torch.cuda.OutOfMemoryError:
+            out = None  # its pools do not fit beside the forest: the log may
         if out is not None:
             return out
     return _log_lists_batched(batch, geometry, theta, mac_type, dehnen_radius_scale)
