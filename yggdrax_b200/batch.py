@@ -370,13 +370,13 @@ def build_interactions_and_neighbors_batched(batch: BatchedTrees, geometry: Batc
     of every set, from one walk over the whole forest: the per-target walk
     (512 sets of 256 to 65,536 particles: 4.6 -> 3.1 ms of GPU time against
     the generation walk and its log's scatter), or for forests it does not serve (tied
-    leaf codes, more than 2^23 nodes) the generation walk."""
+    leaf codes, more than 2^23 nodes) or not as well (many small sets) the
+    generation walk."""
     if mac_type not in _MAC_CODES:
         raise ValueError(f"Unknown mac_type '{mac_type}'")
     if float(dehnen_radius_scale) <= 0.0:
         raise ValueError("dehnen_radius_scale must be > 0")
-    total = batch.total_nodes
-    if total >= 3 and batch.total_leaves > batch.num_sets and 2 * total <= _PAIR_WALK_MAX_NODES:
+    if _takes_target_walk(batch):
         try:
             out = _target_lists_batched(batch, geometry, theta, mac_type, dehnen_radius_scale)
         except torch.cuda.OutOfMemoryError:
@@ -384,6 +384,28 @@ def build_interactions_and_neighbors_batched(batch: BatchedTrees, geometry: Batc
         if out is not None:
             return out
     return _log_lists_batched(batch, geometry, theta, mac_type, dehnen_radius_scale)
+
+
+# Which of the two walks: a target of the per-target walk costs its piece and its
+# place in the queue whatever its lists hold, which the short lists of small sets
+# do not pay for; a generation costs its launches, which a small forest does not
+# pay for.  Call times, per-target against generation walk, leaves of 16,
+# Dehnen's criterion at 0.6 (the line moves little with either):
+#   nodes   nodes per set     37            125           250           375
+#    25,000              264 /   397    262 /   465   304 /   508   295 /   515 us
+#   175,000              437 /   477    540 /   749
+#   250,000              558 /   519    717 /   740   816 /   938   888 / 1,040
+#   500,000                           1,181 /   993
+# 1,000,000            1,596 /   859  2,247 / 1,628 2,607 / 2,467 2,906 / 3,131
+_SMALL_FOREST = 3 << 16   # nodes
+_SMALL_SETS = 300         # nodes per set
+
+
+def _takes_target_walk(batch) -> bool:
+    total, sets = batch.total_nodes, batch.num_sets
+    if total < 3 or batch.total_leaves <= sets or 2 * total > _PAIR_WALK_MAX_NODES:
+        return False
+    return total <= _SMALL_FOREST or total >= _SMALL_SETS * sets
 
 
 # First capacities of a forest's per-target walk, entries per node (far, near
