@@ -12,10 +12,10 @@
 // keys.
 //
 // The sort is what this costs.  A key of more than 64 bits is sorted by its
-// top 64 alone (8 passes of the onesweep sort); the few pairs that tie there
-// without being of one class (2% of a Plummer tree's pairs, runs of at most a
-// few hundred) are ordered by their remaining bits in place, and only a run
-// too long for that sends the whole list through a sort of the low word first.
+// top 64 alone (8 passes of the onesweep sort); the pairs that tie there out of
+// order are ordered by their remaining bits in place (2% of a Plummer tree's
+// pairs, most of a lattice's: GroupTies), and only a run too long for that sends
+// the whole list through a sort of the low word first.
 // Beside the sort, the fields are recomputed where they are needed instead of
 // stored (two 62-byte passes over the pairs became one of 24 bytes), each pair
 // travels as one 16-byte record, and the class tables are decoded from the
@@ -127,10 +127,17 @@ __device__ __forceinline__ void group_fields(const GroupPairs& g, const CellTabl
   }
 }
 
-// Minima / maxima of the fields (for the key widths).
+// Minima / maxima of the fields (for the key widths), a CTA's in shared memory
+// first: with an atomic per warp on the same ten words the kernel waited for them
+// (3.5 M pairs 92 -> 62 us).
 __global__ void k_group_ranges(const GroupPairs g, int* __restrict__ fmin,
                                int* __restrict__ fmax) {
   __shared__ CellTable cells;
+  __shared__ int s_lo[5], s_hi[5];
+  if (threadIdx.x < 5) {
+    s_lo[threadIdx.x] = INT_MAX;
+    s_hi[threadIdx.x] = INT_MIN;
+  }
   cells.fill(g.ext);
   int lo[5], hi[5];
   for (int f = 0; f < 5; ++f) {
@@ -154,9 +161,14 @@ __global__ void k_group_ranges(const GroupPairs g, int* __restrict__ fmin,
       hi[f] = b > hi[f] ? b : hi[f];
     }
     if ((threadIdx.x & 31) == 0) {
-      atomicMin(&fmin[f], lo[f]);
-      atomicMax(&fmax[f], hi[f]);
+      atomicMin(&s_lo[f], lo[f]);
+      atomicMax(&s_hi[f], hi[f]);
     }
+  }
+  __syncthreads();
+  if (threadIdx.x < 5) {
+    atomicMin(&fmin[threadIdx.x], s_lo[threadIdx.x]);
+    atomicMax(&fmax[threadIdx.x], s_hi[threadIdx.x]);
   }
 }
 
@@ -195,47 +207,221 @@ __global__ void k_group_pack(const GroupPairs g, KeyLayout kl, KeyLayout* __rest
   }
 }
 
-// Pairs sorted by `top`: runs of equal words ordered by `low` (stably), out of
-// place.  A warp ranks the runs that start at its 32 positions one after the
-// other, each against itself; runs of more than kTieMax pairs are flagged.
-constexpr int kTieMax = 1024;
-__global__ void k_group_ties(const uint64_t* __restrict__ top, const uint32_t* __restrict__ perm,
-                             const GroupRec* __restrict__ rec, int64_t P,
-                             uint32_t* __restrict__ out, int* __restrict__ too_long) {
+// Pairs sorted by `top` whose runs of equal words are not yet in the order of
+// `low`.  Three kernels, since runs differ: a Plummer tree's hold two to a few
+// hundred pairs of different classes, a lattice's thousands of one or a few.
+//  * k_group_ties copies the order, ranks the runs that lie within a warp's 32
+//    positions, and lists descents of the others (a pair whose `low` is below that
+//    of the pair before it): every run that has any gets one listed, a long one
+//    once in a while.  A run without, such as one class of any size, is in order.
+//  * k_group_short takes the descents, a warp each: the first listed of a run of at
+//    most kTieMax pairs ranks the run against itself; longer runs are listed.
+//  * k_group_long sorts those, a CTA per run, by 8-bit digits of `low`.  A run
+//    longer than GroupTies::longest is flagged: the whole list is then sorted by
+//    `low` first, which costs about what a CTA's sort of 1/64 of it does.
+// Ranking every run, and flagging those past 1,024 pairs, took the grouping of a
+// lattice of 100^3 points, leaf 8 (15.7 M pairs, 65 bits), to 7.5 ms: 2.7 so, and
+// 3.3 with the two sorts of the whole list.  128^3 points, leaf 4 (55.8 M pairs, 76
+// bits): 23.0, 13.8 and 14.2 ms.
+constexpr int kTieMax = 256;
+struct GroupTies {
+  const uint64_t* top;
+  const GroupRec* rec;
+  int64_t P;
+  uint32_t* perm;     // sorted position -> pair, read only until k_group_long
+  uint32_t* out;      // the same in order
+  uint32_t* descents;
+  uint2* runs;        // first position, pairs
+  // one per kTieMax positions, zeroed: no two longer runs start in one (claims),
+  // or reach into it by more than that (seen)
+  uint32_t *claims, *seen;
+  int* count;         // run too long; descents; long runs; long runs taken
+  int64_t longest;
+};
+
+__global__ void k_group_ties(const GroupTies g) {
   const int lane = threadIdx.x & 31;
-  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < P;
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < g.P;
        i0 += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = i0 + lane;
-    int len = 0;
-    if (i < P && (i == 0 || top[i - 1] != top[i])) {
-      const uint64_t w = top[i];
-      len = 1;
-      while (len <= kTieMax && i + len < P && top[i + len] == w) ++len;
-      if (len == 1) out[i] = perm[i];
-      if (len > kTieMax) *too_long = 1;
-    }
-    unsigned runs = __ballot_sync(0xffffffffu, len > 1 && len <= kTieMax);
-    while (runs) {
-      const int from = __ffs(runs) - 1;
-      runs &= runs - 1;
-      const int64_t a = i0 + from;
-      const int n = __shfl_sync(0xffffffffu, len, from);
-      for (int e0 = 0; e0 < n; e0 += 32) {
-        const int e = e0 + lane;
-        const uint32_t mine = e < n ? perm[a + e] : 0u;
-        const uint64_t low = e < n ? rec[mine].low : 0ull;
-        int rank = 0;
-        for (int j0 = 0; j0 < n; j0 += 32) {
-          const uint64_t theirs = j0 + lane < n ? rec[perm[a + j0 + lane]].low : 0ull;
-          const int m = n - j0 < 32 ? n - j0 : 32;
-          for (int j = 0; j < m; ++j) {
-            const uint64_t v = __shfl_sync(0xffffffffu, theirs, j);
-            rank += v < low || (v == low && j0 + j < e);
-          }
-        }
-        if (e < n) out[a + rank] = mine;
+    const bool live = i < g.P;
+    const uint64_t t = live ? g.top[i] : 0ull;
+    const uint32_t p = live ? g.perm[i] : 0u;
+    uint64_t before = __shfl_up_sync(0xffffffffu, t, 1);
+    if (lane == 0 && live && i > 0) before = g.top[i - 1];
+    const bool tied = live && i > 0 && before == t;
+    const unsigned ties = __ballot_sync(0xffffffffu, tied);
+    const bool next = (ties >> lane) & 2u;  // the pair after this one is tied to it
+    const uint64_t low = tied || next ? g.rec[p].low : 0ull;
+    uint64_t low_before = __shfl_up_sync(0xffffffffu, low, 1);
+    if (lane == 0 && tied) low_before = g.rec[g.perm[i - 1]].low;
+    const bool descent = tied && low < low_before;
+    const unsigned m = __ballot_sync(0xffffffffu, descent);
+    int64_t at = i;
+    if (m) {
+      // a run within these 32 positions is ranked here
+      const bool on = lane == 31 && i + 1 < g.P && g.top[i + 1] == t;
+      const unsigned open = __ballot_sync(0xffffffffu, on) ? ~0u : 0u;
+      const unsigned heads = ~ties, upto = heads & (2u * (1u << lane) - 1u);
+      const int start = upto ? 31 - __clz(upto) : -1;  // -1: it comes from before
+      const bool inside = start >= 0 && (!open || (heads & ~(2u * (1u << lane) - 1u)));
+      int rank = 0;
+      for (int j = 0; j < 32; ++j) {
+        const uint64_t v = __shfl_sync(0xffffffffu, low, j);
+        const int s = __shfl_sync(0xffffffffu, start, j);
+        rank += s == start && (v < low || (v == low && j < lane));
       }
+      if (inside) at = i0 + start + rank;
+      // of the others, one descent a run, and one per kTieMax positions further
+      // than that from its run's start
+      const unsigned same = __match_any_sync(0xffffffffu, descent && !inside ? start : 32 + lane);
+      bool list = descent && !inside && lane == __ffs(same) - 1;
+      if (list && i >= kTieMax && g.top[i - kTieMax] == t)
+        list = atomicExch(&g.seen[i / kTieMax], 1u) == 0u;
+      const unsigned ml = __ballot_sync(0xffffffffu, list);
+      int base = 0;
+      if (lane == 0 && ml) base = atomicAdd(&g.count[1], __popc(ml));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (list) g.descents[(uint32_t)base + __popc(ml & ((1u << lane) - 1u))] = (uint32_t)i;
     }
+    if (live) g.out[at] = p;
+  }
+}
+
+// The end of the run that holds position d: how far its word goes on in
+// direction `dir`, found by 31 doublings at once, then by 32 probes a step.
+__device__ __forceinline__ int64_t group_reach(const GroupTies& g, int64_t d, int dir, int lane) {
+  const uint64_t w = g.top[d];
+  auto in = [&](int64_t k) {
+    const int64_t q = d + dir * k;
+    return q >= 0 && q < g.P && g.top[q] == w;
+  };
+  const unsigned m = __ballot_sync(0xffffffffu, lane < 31 && in((int64_t)1 << lane));
+  const int n = __ffs(~m) - 1;  // 2^0 .. 2^(n-1) are in the run
+  int64_t lo = n > 0 ? (int64_t)1 << (n - 1) : 0, hi = (int64_t)1 << n;  // in, out
+  while (hi - lo > 1) {
+    const int64_t step = (hi - lo + 31) / 32, k = lo + step * (lane + 1);
+    const unsigned q = __ballot_sync(0xffffffffu, k < hi && in(k));
+    const int c = __ffs(~q) - 1;  // (bit 31 clear: lo + 32 step >= hi)
+    const int64_t at = lo + step * c;
+    hi = at + step < hi ? at + step : hi;
+    lo = at;
+  }
+  return lo;
+}
+
+__global__ void k_group_short(const GroupTies g) {
+  const int lane = threadIdx.x & 31;
+  const int warps = (int)(gridDim.x * blockDim.x) >> 5;
+  const uint32_t n_desc = (uint32_t)g.count[1];
+  for (uint32_t e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < n_desc; e += warps) {
+    const int64_t d = g.descents[e];
+    const int64_t a = d - group_reach(g, d, -1, lane), n = d - a + group_reach(g, d, 1, lane) + 1;
+    if (n > kTieMax) {
+      if (lane == 0 && atomicExch(&g.claims[a / kTieMax], 1u) == 0u) {
+        if (n > g.longest) g.count[0] = 1;
+        else g.runs[atomicAdd(&g.count[2], 1)] = make_uint2((uint32_t)a, (uint32_t)n);
+      }
+      continue;
+    }
+    // the run's first descent?  (the first is listed: it is its warp's first of
+    // the run, and less than kTieMax behind the run's start)
+    bool first = true;
+    for (int64_t q0 = a; q0 + 1 < d && first; q0 += 31) {
+      const int64_t q = q0 + lane;
+      const uint64_t low = q < d ? g.rec[g.perm[q]].low : ~0ull;
+      const uint64_t next = __shfl_down_sync(0xffffffffu, low, 1);
+      first = !__any_sync(0xffffffffu, lane < 31 && next < low);
+    }
+    if (!first) continue;
+    for (int e0 = 0; e0 < n; e0 += 32) {
+      const int k = e0 + lane;
+      const uint32_t mine = k < n ? g.perm[a + k] : 0u;
+      const uint64_t low = k < n ? g.rec[mine].low : 0ull;
+      int rank = 0;
+      for (int j0 = 0; j0 < n; j0 += 32) {
+        const uint64_t theirs = j0 + lane < n ? g.rec[g.perm[a + j0 + lane]].low : 0ull;
+        const int m = n - j0 < 32 ? (int)(n - j0) : 32;
+        for (int j = 0; j < m; ++j) {
+          const uint64_t v = __shfl_sync(0xffffffffu, theirs, j);
+          rank += v < low || (v == low && j0 + j < k);
+        }
+      }
+      if (k < n) g.out[a + rank] = mine;
+    }
+  }
+}
+
+// Least digit first, stable: the run's histogram, then its pairs 512 at a time,
+// each at its digit's place plus its rank among the chunk's.  A digit that all
+// pairs share moves nothing.
+constexpr int kLongThreads = 512;
+constexpr int kLongWarps = kLongThreads / 32;
+__global__ void __launch_bounds__(kLongThreads) k_group_long(const GroupTies g, int cut) {
+  __shared__ uint32_t s_bin[256], s_all[256];
+  __shared__ uint16_t s_warp[kLongWarps][256];
+  __shared__ uint32_t s_run;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t n_runs = (uint32_t)g.count[2];
+  while (true) {
+    if (tid == 0) s_run = (uint32_t)atomicAdd(&g.count[3], 1);
+    __syncthreads();
+    if (s_run >= n_runs) break;
+    const uint2 run = g.runs[s_run];
+    const uint32_t n = run.y;
+    uint32_t *src = g.perm + run.x, *dst = g.out + run.x;
+    for (int shift = 0; shift < cut; shift += 8) {
+      auto digit = [&](uint32_t p) { return (int)(g.rec[p].low >> shift) & 255; };
+      if (tid < 256) s_bin[tid] = 0u;
+      __syncthreads();
+      for (uint32_t k = tid; k < n; k += kLongThreads) atomicAdd(&s_bin[digit(__ldcg(src + k))], 1u);
+      __syncthreads();
+      if (__syncthreads_or(tid < 256 && s_bin[tid] == n)) continue;
+      if (warp == 0) {  // exclusive sums, 8 digits a lane
+        uint32_t v[8], sum = 0;
+        for (int j = 0; j < 8; ++j) {
+          v[j] = sum;
+          sum += s_bin[8 * lane + j];
+        }
+        uint32_t incl = sum;
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t w = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += w;
+        }
+        for (int j = 0; j < 8; ++j) s_bin[8 * lane + j] = incl - sum + v[j];
+      }
+      for (uint32_t c0 = 0; c0 < n; c0 += kLongThreads) {
+        for (int k = tid; k < kLongWarps * 256; k += kLongThreads) (&s_warp[0][0])[k] = 0;
+        __syncthreads();
+        const uint32_t k = c0 + tid;
+        const uint32_t p = k < n ? __ldcg(src + k) : 0u;
+        const int d = k < n ? digit(p) : 256;
+        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        const int rank = __popc(peers & ((1u << lane) - 1u));
+        if (k < n && rank == 0) s_warp[warp][d] = (uint16_t)__popc(peers);
+        __syncthreads();
+        if (tid < 256) {
+          uint32_t sum = 0;  // counts of the warps before, and the chunk's
+          for (int w = 0; w < kLongWarps; ++w) {
+            const uint32_t c = s_warp[w][tid];
+            s_warp[w][tid] = (uint16_t)sum;
+            sum += c;
+          }
+          s_all[tid] = sum;
+        }
+        __syncthreads();
+        if (k < n) dst[s_bin[d] + s_warp[warp][d] + rank] = p;
+        __syncthreads();
+        if (tid < 256) s_bin[tid] += s_all[tid];
+      }
+      __syncthreads();
+      uint32_t* x = src;
+      src = dst;
+      dst = x;
+    }
+    if (src == g.perm + run.x)  // nothing moved (out holds the copy), or an even number of times
+      for (uint32_t k = tid; k < n; k += kLongThreads) dst[k] = __ldcg(src + k);
+    __syncthreads();
   }
 }
 
@@ -351,7 +537,7 @@ __global__ void __launch_bounds__(kScanThreads)
 struct GroupScratch {
   int* fmin;
   int* fmax;
-  int* too_long;
+  int* too_long;         // GroupTies::count
   KeyLayout* layout;
   uint64_t* top;         // pair order
   uint64_t* top_sorted;
@@ -383,8 +569,8 @@ GroupScratch carve_group(Arena& a, int64_t P) {
   return g;
 }
 
-__global__ void k_init_minmax(int* fmin, int* fmax, int* too_long) {
-  if (threadIdx.x == 0) *too_long = 0;
+__global__ void k_init_minmax(int* fmin, int* fmax, int* too_long) {  // (GroupTies::count)
+  if (threadIdx.x < 4) too_long[threadIdx.x] = 0;
   if (threadIdx.x < 5) {
     fmin[threadIdx.x] = INT_MAX;
     fmax[threadIdx.x] = INT_MIN;
@@ -498,9 +684,27 @@ int ygx_grouped_classes(const void* sources, const void* targets, int index_bits
                               stream);
       if (rc) return rc;
       if (kl.cut) {
-        ygx::k_group_ties<<<ygx::grid_for(P, 256), 256, 0, stream>>>(g.top_sorted, g.perm_a, g.rec,
-                                                                     P, g.perm_b, g.too_long);
+        // the lists lie where the heads' records come, 16 bytes a pair: at most P
+        // descents, P / kTieMax runs, twice P / kTieMax + 1 words (P > 1 here: one
+        // pair's key has no bits)
+        char* lists = reinterpret_cast<char*>(g.rec_sorted);
+        uint32_t* claims = reinterpret_cast<uint32_t*>(lists + 12 * P);
+        const int64_t blocks = P / ygx::kTieMax + 1;
+        if (cudaMemsetAsync(claims, 0, 2 * sizeof(uint32_t) * blocks, stream) != cudaSuccess)
+          return YGX_ERR_CUDA;
+        const ygx::GroupTies ties{g.top_sorted, g.rec, P, g.perm_a, g.perm_b,
+                                  reinterpret_cast<uint32_t*>(lists),
+                                  reinterpret_cast<uint2*>(lists + 4 * (P + P % 2)),
+                                  claims, claims + blocks, g.too_long,
+                                  P / 64 > 16384 ? P / 64 : 16384};
+        ygx::k_group_ties<<<ygx::grid_for(P, 256), 256, 0, stream>>>(ties);
         YGX_CHECK_LAUNCH();
+        ygx::k_group_short<<<ygx::grid_for(P, 256), 256, 0, stream>>>(ties);
+        YGX_CHECK_LAUNCH();
+        if (P > ygx::kTieMax) {
+          ygx::k_group_long<<<ygx::kNumSMs * 2, ygx::kLongThreads, 0, stream>>>(ties, kl.cut);
+          YGX_CHECK_LAUNCH();
+        }
       }
     } else {
       uint64_t* keys = reinterpret_cast<uint64_t*>(g.rec_sorted);  // free until the heads
