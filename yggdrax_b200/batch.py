@@ -300,7 +300,10 @@ def compute_tree_geometry_batched(batch: BatchedTrees) -> BatchedGeometry:
 @dataclass
 class BatchedInteractions:
     """Far / near lists of every set, packed: far rows in level-major order
-    set after set, near rows leaf by leaf; node ids local to each set."""
+    set after set, near rows leaf by leaf; node ids local to each set.
+    ``stats``: totals, longest rows, decisions, generations and largest
+    wavefront of the walk; ``wf_need`` and ``log_need`` are sizes of the
+    generation walk's own buffers, 0 where the per-target walk ran."""
 
     node_offsets: torch.Tensor   # (total+1,) global row starts, node-indexed
     far_counts: torch.Tensor
