@@ -707,7 +707,8 @@ int ygx_tree_moments(const float* positions_sorted, const float* masses_sorted, 
  * (host) = far and near pairs the lists would hold (counted past the
  * capacities); flags_out (host): bit 0 far, bit 1 near, bit 2 wavefront
  * (max_pair_queue) overflow -- the walk stops after the generation that set
- * one, like the reference.  Synchronizes once per generation. */
+ * one, like the reference.  All generations run in one launch; synchronizes
+ * once. */
 size_t ygx_mutual_walk_workspace_size(int64_t total, int64_t max_pair_queue);
 int ygx_mutual_walk(const void* left_full, const void* right_full, int index_bits,
                     const float* centers, const float* radii, int64_t total, float theta,
@@ -760,8 +761,8 @@ int ygx_octree_view(const uint8_t* valid, const uint8_t* leaf, const uint64_t* c
  * max_pair_queue (the walk stops after that generation, like the reference),
  * bit 4 more children than wf_capacity (re-run with stats_out[6] or more),
  * bit 5 the log was too short (the walk ran on; re-run with stats_out[0] or
- * [1] entries).  Synchronizes once per
- * generation.  A stable sort of the log by key gives the reference's rows. */
+ * [1] entries).  All generations run in one launch; synchronizes once.  A
+ * stable sort of the log by key gives the reference's rows. */
 size_t ygx_octree_walk_workspace_size(int64_t M, int64_t wf_capacity);
 int ygx_octree_walk(const void* children, const void* child_counts, int index_bits, int64_t M,
                     const float* centers, const float* radii, const float* max_extents,

@@ -92,7 +92,8 @@ struct TwBlkSet {
   TwBlk far, near_, s, far_r, near_r, s_r;
 };
 // A warp's counters (lane 0 only): decisions per side, cycles on pieces and
-// waiting, pieces, 32-wide steps and the candidates they held.
+// waiting, pieces, steps (32 candidates wide in k_tw_walk, 64 in k_pair_walk)
+// and the candidates they held.
 struct TwWarpStats {
   unsigned long long acc, near_, ref, busy, idle, pieces, steps, lanes;
 };
@@ -135,7 +136,7 @@ struct __align__(128) TwCtl {
   // written once per warp at exit
   unsigned long long acc_sides, near_sides, ref_sides;  // decision counts (per side)
   unsigned long long busy_cycles, idle_cycles, pieces;  // where the warps' time went
-  unsigned long long steps, lanes;  // 32-wide steps run, candidates they held
+  unsigned long long steps, lanes;  // steps run, candidates they held
   unsigned int max_cmp;                                 // most chunks of one split list
   unsigned int pad[3];
 };
