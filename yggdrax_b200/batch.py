@@ -379,36 +379,70 @@ def build_interactions_and_neighbors_batched(batch: BatchedTrees, geometry: Batc
         raise ValueError(f"Unknown mac_type '{mac_type}'")
     if float(dehnen_radius_scale) <= 0.0:
         raise ValueError("dehnen_radius_scale must be > 0")
-    if _takes_target_walk(batch):
+    total = batch.total_nodes
+    expected = _expected_entries(total, batch.num_sets, batch.leaf_size, mac_type, float(theta),
+                                 float(dehnen_radius_scale))
+    key = _hint_key(mac_type, theta, total, "batch_entries")
+    out = None
+    if _takes_target_walk(batch, expected, key):
         try:
             out = _target_lists_batched(batch, geometry, theta, mac_type, dehnen_radius_scale)
         except torch.cuda.OutOfMemoryError:
-            out = None  # its pools do not fit beside the forest: the log may
-        if out is not None:
-            return out
-    return _log_lists_batched(batch, geometry, theta, mac_type, dehnen_radius_scale)
+            pass  # its pools do not fit beside the forest: the log may
+    if out is None:
+        out = _log_lists_batched(batch, geometry, theta, mac_type, dehnen_radius_scale)
+    if out.stats:
+        entries = (out.stats["far_total"] + out.stats["near_total"]) / total
+        _ENTRIES_HINTS[key] = entries / expected
+    return out
 
 
 # Which of the two walks: a target of the per-target walk costs its piece and its
-# place in the queue whatever its lists hold, which the short lists of small sets
-# do not pay for; a generation costs its launches, which a small forest does not
-# pay for.  Call times, per-target against generation walk, leaves of 16,
-# Dehnen's criterion at 0.6 (the line moves little with either):
-#   nodes   nodes per set     37            125           250           375
+# place in the queue whatever its lists hold, which short lists do not pay for; a
+# generation costs its launches, which a small forest does not pay for, and its log's
+# scatter, which a large one pays most for.  So the line is a length of lists, which
+# rises with the forest to 64 entries per node at 1 M nodes and falls behind them.  Call times, per-target
+# against generation walk (leaves of 16, Dehnen's criterion at 0.6; sets of 37, 125,
+# 250 and 375 nodes):
+#   nodes   entries per node   9             31            55            71
 #    25,000              264 /   397    262 /   465   304 /   508   295 /   515 us
 #   175,000              437 /   477    540 /   749
 #   250,000              558 /   519    717 /   740   816 /   938   888 / 1,040
 #   500,000                           1,181 /   993
 # 1,000,000            1,596 /   859  2,247 / 1,628 2,607 / 2,467 2,906 / 3,131
-_SMALL_FOREST = 3 << 16   # nodes
-_SMALL_SETS = 300         # nodes per set
+# 2,750,000 (Barnes-Hut at 0.5)                            7,206 / 8,532
+# 3,600,000 (Plummer-like sets, 0.8)                      10,230 / 12,951
+# Points on a line, leaves of 4, 1.5 M nodes, 3 entries: 2,799 / 1,200.  Over 140
+# forests of 90,000 to 4 M nodes, 8 to 4,096 of them per set, leaves of 1 to 32,
+# cubes, balls, clumps and lines, the walk taken was 2.8% slower than the better one
+# on average when first met (the lines), 0.3% after that.
+_SMALL_FOREST = 3 << 16  # nodes
+_LINE_ENTRIES = 80.0     # entries per node
+# Entries per node of a set of many nodes at theta 0.6 in leaves of 16 and more, as
+# counted on uniform cubes.
+_SET_ENTRIES = {"bh": 70.0, "dehnen": 190.0, "engblom": 85.0}
+# Entries that the last forest of a kind had, against what was expected of it: points
+# on a line have a tenth.  Per (criterion, theta, size octave).
+_ENTRIES_HINTS: dict = {}
 
 
-def _takes_target_walk(batch) -> bool:
+def _expected_entries(total: int, sets: int, leaf_size: int, mac_type: str, theta: float,
+                      scale: float) -> float:
+    """Entries per node: a set's lists are all its pairs while it is small, and
+    the sphere of 1 / theta around a node, which leaves of few points fill less."""
+    nodes = total / sets
+    if not theta > 0.0:
+        return nodes / 3.2
+    full = _SET_ENTRIES[mac_type] * (0.6 * scale / theta) ** 3 * max(0.1, 1.0 - 1.0 / leaf_size)
+    return full * nodes / (nodes + 3.2 * full)
+
+
+def _takes_target_walk(batch, expected: float, key) -> bool:
     total, sets = batch.total_nodes, batch.num_sets
     if total < 3 or batch.total_leaves <= sets or 2 * total > _PAIR_WALK_MAX_NODES:
         return False
-    return total <= _SMALL_FOREST or total >= _SMALL_SETS * sets
+    line = _LINE_ENTRIES * (1.0 - _SMALL_FOREST / total) * min(1.0, (2 ** 20 / total) ** 0.5)
+    return expected * _ENTRIES_HINTS.get(key, 1.0) >= line
 
 
 # First capacities of a forest's per-target walk, entries per node (far, near
