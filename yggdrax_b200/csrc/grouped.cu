@@ -14,8 +14,7 @@
 // The sort is what this costs.  A key of more than 64 bits is sorted by its
 // top 64 alone (8 passes of the onesweep sort); the pairs that tie there out of
 // order are ordered by their remaining bits in place (2% of a Plummer tree's
-// pairs, most of a lattice's: GroupTies), and only a run too long for that sends
-// the whole list through a sort of the low word first.
+// pairs, most of a lattice's: GroupTies).  A few bits more than 64 are sorted first.
 // Beside the sort, the fields are recomputed where they are needed instead of
 // stored (two 62-byte passes over the pairs became one of 24 bytes), each pair
 // travels as one 16-byte record, and the class tables are decoded from the
@@ -216,13 +215,13 @@ __global__ void k_group_pack(const GroupPairs g, KeyLayout kl, KeyLayout* __rest
 //    once in a while.  A run without, such as one class of any size, is in order.
 //  * k_group_short takes the descents, a warp each: the first listed of a run of at
 //    most kTieMax pairs ranks the run against itself; longer runs are listed.
-//  * k_group_long sorts those, a CTA per run, by 8-bit digits of `low`.  A run
-//    longer than GroupTies::longest is flagged: the whole list is then sorted by
-//    `low` first, which costs about what a CTA's sort of 1/64 of it does.
-// Ranking every run, and flagging those past 1,024 pairs, took the grouping of a
-// lattice of 100^3 points, leaf 8 (15.7 M pairs, 65 bits), to 7.5 ms: 2.7 so, and
-// 3.3 with the two sorts of the whole list.  128^3 points, leaf 4 (55.8 M pairs, 76
-// bits): 23.0, 13.8 and 14.2 ms.
+//  * k_group_long sorts those, a CTA per run, by 8-bit digits of `low`.  Runs
+//    longer than 1/64 of the list (fewer than 64 there are) go through the onesweep
+//    sort one by one: a CTA's sort of so many pairs costs what the passes over the
+//    whole list do.
+// Ranking every run, and sorting the whole list twice more if one was longer than
+// 1,024 pairs, took the grouping of a lattice of 128^3 points, leaf 4 (55.8 M pairs,
+// 76 bits), to 23.0 ms; 13.4 so.
 constexpr int kTieMax = 256;
 struct GroupTies {
   const uint64_t* top;
@@ -235,9 +234,17 @@ struct GroupTies {
   // one per kTieMax positions, zeroed: no two longer runs start in one (claims),
   // or reach into it by more than that (seen)
   uint32_t *claims, *seen;
-  int* count;         // run too long; descents; long runs; long runs taken
+  int* count;         // huge runs; descents; long runs; long runs taken
+  uint2* huge;        // kHugeRuns: runs of more than `longest` pairs
   int64_t longest;
 };
+constexpr int kHugeRuns = 64;
+// Up to this many bits below the top word, one pass, are sorted first instead: the
+// pass, its keys and the gather of the top words cost what a look at the ties does
+// (37 M jittered lattice pairs, 71 bits: 7.0 ms the call, 6.4 with the ties) and
+// nothing more where many tie (11 M pairs of 60,000 points of which a third coincide,
+// 67 bits: 2.1 and 2.5).  Two passes cost a Plummer tree twice its ties.
+constexpr int kLowFirst = 8;
 
 __global__ void k_group_ties(const GroupTies g) {
   const int lane = threadIdx.x & 31;
@@ -319,7 +326,7 @@ __global__ void k_group_short(const GroupTies g) {
     const int64_t a = d - group_reach(g, d, -1, lane), n = d - a + group_reach(g, d, 1, lane) + 1;
     if (n > kTieMax) {
       if (lane == 0 && atomicExch(&g.claims[a / kTieMax], 1u) == 0u) {
-        if (n > g.longest) g.count[0] = 1;
+        if (n > g.longest) g.huge[atomicAdd(&g.count[0], 1)] = make_uint2((uint32_t)a, (uint32_t)n);
         else g.runs[atomicAdd(&g.count[2], 1)] = make_uint2((uint32_t)a, (uint32_t)n);
       }
       continue;
@@ -352,11 +359,14 @@ __global__ void k_group_short(const GroupTies g) {
   }
 }
 
-// Least digit first, stable: the run's histogram, then its pairs 512 at a time,
-// each at its digit's place plus its rank among the chunk's.  A digit that all
-// pairs share moves nothing.
+// Least digit first, stable: the run's histogram, then its pairs 4,096 at a time --
+// 256 a warp, eight of its lanes' in flight --, each at its digit's place plus its
+// rank among the chunk's.  A digit that all pairs share moves nothing.  Bound by the
+// gathers of `low` and the chunks' barriers: 140,000 pairs, one digit, 409 us with
+// 512 at a time, 234 so.
 constexpr int kLongThreads = 512;
 constexpr int kLongWarps = kLongThreads / 32;
+constexpr int kLongItems = 8;
 __global__ void __launch_bounds__(kLongThreads) k_group_long(const GroupTies g, int cut) {
   __shared__ uint32_t s_bin[256], s_all[256];
   __shared__ uint16_t s_warp[kLongWarps][256];
@@ -374,7 +384,18 @@ __global__ void __launch_bounds__(kLongThreads) k_group_long(const GroupTies g, 
       auto digit = [&](uint32_t p) { return (int)(g.rec[p].low >> shift) & 255; };
       if (tid < 256) s_bin[tid] = 0u;
       __syncthreads();
-      for (uint32_t k = tid; k < n; k += kLongThreads) atomicAdd(&s_bin[digit(__ldcg(src + k))], 1u);
+      for (uint32_t k = tid; k < n; k += kLongThreads * 4) {
+        uint32_t p[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          p[u] = k + u * kLongThreads < n ? __ldcg(src + k + u * kLongThreads) : 0u;
+        int d[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) d[u] = digit(p[u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (k + u * kLongThreads < n) atomicAdd(&s_bin[d[u]], 1u);
+      }
       __syncthreads();
       if (__syncthreads_or(tid < 256 && s_bin[tid] == n)) continue;
       if (warp == 0) {  // exclusive sums, 8 digits a lane
@@ -390,15 +411,27 @@ __global__ void __launch_bounds__(kLongThreads) k_group_long(const GroupTies g, 
         }
         for (int j = 0; j < 8; ++j) s_bin[8 * lane + j] = incl - sum + v[j];
       }
-      for (uint32_t c0 = 0; c0 < n; c0 += kLongThreads) {
+      for (uint32_t c0 = 0; c0 < n; c0 += kLongThreads * kLongItems) {
         for (int k = tid; k < kLongWarps * 256; k += kLongThreads) (&s_warp[0][0])[k] = 0;
+        const uint32_t k0 = c0 + warp * (32 * kLongItems) + lane;
+        uint32_t p[kLongItems];
+        int d[kLongItems];
+        uint16_t rank[kLongItems];
+#pragma unroll
+        for (int u = 0; u < kLongItems; ++u) p[u] = k0 + 32 * u < n ? __ldcg(src + k0 + 32 * u) : 0u;
+#pragma unroll
+        for (int u = 0; u < kLongItems; ++u) d[u] = k0 + 32 * u < n ? digit(p[u]) : 256;
         __syncthreads();
-        const uint32_t k = c0 + tid;
-        const uint32_t p = k < n ? __ldcg(src + k) : 0u;
-        const int d = k < n ? digit(p) : 256;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        const int rank = __popc(peers & ((1u << lane) - 1u));
-        if (k < n && rank == 0) s_warp[warp][d] = (uint16_t)__popc(peers);
+#pragma unroll
+        for (int u = 0; u < kLongItems; ++u) {
+          const unsigned peers = __match_any_sync(0xffffffffu, d[u]);
+          const int before = __popc(peers & ((1u << lane) - 1u));
+          const uint16_t held = d[u] < 256 ? s_warp[warp][d[u]] : (uint16_t)0;
+          rank[u] = (uint16_t)(held + before);
+          __syncwarp();
+          if (d[u] < 256 && before == 0) s_warp[warp][d[u]] = (uint16_t)(held + __popc(peers));
+          __syncwarp();
+        }
         __syncthreads();
         if (tid < 256) {
           uint32_t sum = 0;  // counts of the warps before, and the chunk's
@@ -410,7 +443,9 @@ __global__ void __launch_bounds__(kLongThreads) k_group_long(const GroupTies g, 
           s_all[tid] = sum;
         }
         __syncthreads();
-        if (k < n) dst[s_bin[d] + s_warp[warp][d] + rank] = p;
+#pragma unroll
+        for (int u = 0; u < kLongItems; ++u)
+          if (d[u] < 256) dst[s_bin[d[u]] + s_warp[warp][d[u]] + rank[u]] = p[u];
         __syncthreads();
         if (tid < 256) s_bin[tid] += s_all[tid];
       }
@@ -437,6 +472,13 @@ __global__ void k_gather_u64(const uint64_t* __restrict__ in, const uint32_t* __
        i += (int64_t)gridDim.x * blockDim.x)
     out[i] = in[perm[i]];
 }
+__global__ void k_group_run_keys(const GroupRec* __restrict__ rec,
+                                 const uint32_t* __restrict__ perm, int64_t n,
+                                 uint64_t* __restrict__ out) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x)
+    out[i] = rec[perm[i]].low;
+}
 
 // Records in sorted order and the run starts (classes), with the number of
 // runs that start in each tile.
@@ -445,8 +487,7 @@ __global__ void __launch_bounds__(kScanThreads)
                   const GroupRec* __restrict__ rec, int64_t P, GroupRec* __restrict__ sorted,
                   uint8_t* __restrict__ head, int64_t* __restrict__ tile_heads,
                   const int* __restrict__ skip) {
-  // a run too long to order in place has no permutation here (its entries of
-  // `perm` were not written)
+  // a huge run is not in order yet
   if (skip && *skip) return;
   __shared__ int64_t s_warp[kScanThreads / 32];
   const int lane = threadIdx.x & 31;
@@ -537,7 +578,8 @@ __global__ void __launch_bounds__(kScanThreads)
 struct GroupScratch {
   int* fmin;
   int* fmax;
-  int* too_long;         // GroupTies::count
+  int* counts;           // GroupTies::count
+  uint2* huge;           // GroupTies::huge
   KeyLayout* layout;
   uint64_t* top;         // pair order
   uint64_t* top_sorted;
@@ -555,7 +597,8 @@ GroupScratch carve_group(Arena& a, int64_t P) {
   const int64_t n = P > 0 ? P : 1;
   g.fmin = a.take<int>(8);
   g.fmax = a.take<int>(8);
-  g.too_long = a.take<int>(8);
+  g.counts = a.take<int>(8);
+  g.huge = a.take<uint2>(kHugeRuns);
   g.layout = a.take<KeyLayout>(1);
   g.top = a.take<uint64_t>(n);
   g.top_sorted = a.take<uint64_t>(n);
@@ -569,8 +612,8 @@ GroupScratch carve_group(Arena& a, int64_t P) {
   return g;
 }
 
-__global__ void k_init_minmax(int* fmin, int* fmax, int* too_long) {  // (GroupTies::count)
-  if (threadIdx.x < 4) too_long[threadIdx.x] = 0;
+__global__ void k_init_minmax(int* fmin, int* fmax, int* counts) {
+  if (threadIdx.x < 4) counts[threadIdx.x] = 0;
   if (threadIdx.x < 5) {
     fmin[threadIdx.x] = INT_MAX;
     fmax[threadIdx.x] = INT_MIN;
@@ -642,7 +685,7 @@ int ygx_grouped_classes(const void* sources, const void* targets, int index_bits
   const ygx::GroupPairs pairs{sources, targets, index_bits,
                               P,       level32, center,
                               {root_extent[0], root_extent[1], root_extent[2]}};
-  ygx::k_init_minmax<<<1, 32, 0, stream>>>(g.fmin, g.fmax, g.too_long);
+  ygx::k_init_minmax<<<1, 32, 0, stream>>>(g.fmin, g.fmax, g.counts);
   YGX_CHECK_LAUNCH();
   ygx::k_group_ranges<<<ygx::grid_for(P, 256), 256, 0, stream>>>(pairs, g.fmin, g.fmax);
   YGX_CHECK_LAUNCH();
@@ -672,41 +715,14 @@ int ygx_grouped_classes(const void* sources, const void* targets, int index_bits
   const int64_t tiles = ygx::scan_tiles(P);
   struct {
     int64_t classes;
-    int too_long;
+    int huge;
   } h{0, 0};
   // sorted by `top` (one class: the identity order), ties resolved into perm_b;
-  // then, if a run was too long for that, again from a sort by `low`
+  // then, if there are huge runs, again after those
+  const bool ties_later = kl.cut > ygx::kLowFirst;
   for (int attempt = 0; attempt < 2; ++attempt) {
     int rc;
-    if (attempt == 0) {
-      rc = ygx::onesweep_sort(g.top, nullptr, P, 0, bits == 0 ? 1 : (bits > 64 ? 64 : bits),
-                              g.top_sorted, kl.cut ? g.perm_a : g.perm_b, g.sort, false, status,
-                              stream);
-      if (rc) return rc;
-      if (kl.cut) {
-        // the lists lie where the heads' records come, 16 bytes a pair: at most P
-        // descents, P / kTieMax runs, twice P / kTieMax + 1 words (P > 1 here: one
-        // pair's key has no bits)
-        char* lists = reinterpret_cast<char*>(g.rec_sorted);
-        uint32_t* claims = reinterpret_cast<uint32_t*>(lists + 12 * P);
-        const int64_t blocks = P / ygx::kTieMax + 1;
-        if (cudaMemsetAsync(claims, 0, 2 * sizeof(uint32_t) * blocks, stream) != cudaSuccess)
-          return YGX_ERR_CUDA;
-        const ygx::GroupTies ties{g.top_sorted, g.rec, P, g.perm_a, g.perm_b,
-                                  reinterpret_cast<uint32_t*>(lists),
-                                  reinterpret_cast<uint2*>(lists + 4 * (P + P % 2)),
-                                  claims, claims + blocks, g.too_long,
-                                  P / 64 > 16384 ? P / 64 : 16384};
-        ygx::k_group_ties<<<ygx::grid_for(P, 256), 256, 0, stream>>>(ties);
-        YGX_CHECK_LAUNCH();
-        ygx::k_group_short<<<ygx::grid_for(P, 256), 256, 0, stream>>>(ties);
-        YGX_CHECK_LAUNCH();
-        if (P > ygx::kTieMax) {
-          ygx::k_group_long<<<ygx::kNumSMs * 2, ygx::kLongThreads, 0, stream>>>(ties, kl.cut);
-          YGX_CHECK_LAUNCH();
-        }
-      }
-    } else {
+    if (attempt == 0 && kl.cut > 0 && !ties_later) {
       uint64_t* keys = reinterpret_cast<uint64_t*>(g.rec_sorted);  // free until the heads
       ygx::k_group_low_keys<<<ygx::grid_for(P, 256), 256, 0, stream>>>(g.rec, P, keys);
       YGX_CHECK_LAUNCH();
@@ -718,10 +734,55 @@ int ygx_grouped_classes(const void* sources, const void* targets, int index_bits
       rc = ygx::onesweep_sort(keys, g.perm_a, P, 0, 64, g.top_sorted, g.perm_b, g.sort, false,
                               status, stream);
       if (rc) return rc;
+    } else if (attempt == 0) {
+      rc = ygx::onesweep_sort(g.top, nullptr, P, 0, bits == 0 ? 1 : (bits > 64 ? 64 : bits),
+                              g.top_sorted, ties_later ? g.perm_a : g.perm_b, g.sort, false,
+                              status, stream);
+      if (rc) return rc;
+      if (ties_later) {
+        // the lists lie where the heads' records come, 16 bytes a pair: at most P
+        // descents, P / kTieMax runs, twice P / kTieMax + 1 words (P > 1 here: one
+        // pair's key has no bits)
+        char* lists = reinterpret_cast<char*>(g.rec_sorted);
+        uint32_t* claims = reinterpret_cast<uint32_t*>(lists + 12 * P);
+        const int64_t blocks = P / ygx::kTieMax + 1;
+        if (cudaMemsetAsync(claims, 0, 2 * sizeof(uint32_t) * blocks, stream) != cudaSuccess)
+          return YGX_ERR_CUDA;
+        const ygx::GroupTies ties{g.top_sorted, g.rec, P, g.perm_a, g.perm_b,
+                                  reinterpret_cast<uint32_t*>(lists),
+                                  reinterpret_cast<uint2*>(lists + 4 * (P + P % 2)),
+                                  claims, claims + blocks, g.counts, g.huge,
+                                  P / 64 > 16384 ? P / 64 : 16384};
+        ygx::k_group_ties<<<ygx::grid_for(P, 256), 256, 0, stream>>>(ties);
+        YGX_CHECK_LAUNCH();
+        ygx::k_group_short<<<ygx::grid_for(P, 256), 256, 0, stream>>>(ties);
+        YGX_CHECK_LAUNCH();
+        if (P > ygx::kTieMax) {
+          ygx::k_group_long<<<ygx::kNumSMs * 2, ygx::kLongThreads, 0, stream>>>(ties, kl.cut);
+          YGX_CHECK_LAUNCH();
+        }
+      }
+    } else {
+      uint2 runs[ygx::kHugeRuns];
+      if (h.huge > ygx::kHugeRuns ||
+          cudaMemcpyAsync(runs, g.huge, sizeof(uint2) * h.huge, cudaMemcpyDeviceToHost, stream) !=
+              cudaSuccess ||
+          cudaStreamSynchronize(stream) != cudaSuccess)
+        return YGX_ERR_CUDA;
+      uint64_t* keys = reinterpret_cast<uint64_t*>(g.rec_sorted);  // free until the heads
+      for (int k = 0; k < h.huge; ++k) {
+        const int64_t n = runs[k].y;
+        const uint32_t* in = g.perm_a + runs[k].x;
+        ygx::k_group_run_keys<<<ygx::grid_for(n, 256), 256, 0, stream>>>(g.rec, in, n, keys);
+        YGX_CHECK_LAUNCH();
+        rc = ygx::onesweep_sort(keys, in, n, 0, kl.cut, keys + P, g.perm_b + runs[k].x, g.sort,
+                                false, status, stream);
+        if (rc) return rc;
+      }
     }
     ygx::k_group_heads<<<(unsigned)tiles, ygx::kScanThreads, 0, stream>>>(
         g.top_sorted, g.perm_b, g.rec, P, g.rec_sorted, g.head, g.tile_heads,
-        attempt == 0 ? g.too_long : nullptr);
+        attempt == 0 ? g.counts : nullptr);
     YGX_CHECK_LAUNCH();
     // exclusive over the tiles and, as one more "tile", the total
     if (cudaMemsetAsync(g.tile_heads + tiles, 0, sizeof(int64_t), stream) != cudaSuccess)
@@ -730,13 +791,12 @@ int ygx_grouped_classes(const void* sources, const void* targets, int index_bits
     YGX_CHECK_LAUNCH();
     if (cudaMemcpyAsync(&h.classes, g.tile_heads + tiles, sizeof(int64_t), cudaMemcpyDeviceToHost,
                         stream) != cudaSuccess ||
-        (kl.cut && attempt == 0 &&
-         cudaMemcpyAsync(&h.too_long, g.too_long, sizeof(int), cudaMemcpyDeviceToHost, stream) !=
+        (ties_later && attempt == 0 &&
+         cudaMemcpyAsync(&h.huge, g.counts, sizeof(int), cudaMemcpyDeviceToHost, stream) !=
              cudaSuccess) ||
         cudaStreamSynchronize(stream) != cudaSuccess)
       return YGX_ERR_CUDA;
-    if (!h.too_long) break;
-    h.too_long = 0;
+    if (attempt > 0 || !h.huge) break;
   }
   *num_classes_out = h.classes;
   return YGX_OK;
